@@ -46,6 +46,11 @@ __device__ __forceinline__ void st_relaxed64(unsigned long long *p, unsigned lon
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// Release / acquire fence at device scope.  Enough wherever one thread's
+// writes are handed to another through an atomic or a flag; __threadfence()
+// is the sequentially consistent one and measured slower.
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 // Grid-wide barrier for a cooperative (co-resident) launch.  Arrivals count
 // up in *count; the last arrival resets it and bumps *gen.  Waiters spin on
 // *gen with a wall-clock limit; on timeout *err is set and false returned,

@@ -72,10 +72,13 @@ struct alignas(128) PeelQueue {
     unsigned long long pad1[15];
 };
 
+// The end of a level, announced: level index << 32 | next level.
+struct alignas(128) PeelDone {
+    unsigned long long word;
+};
+
 struct PeelCtl {
     unsigned long long pending[3];   // outstanding work credits of level i
-    unsigned long long scan_cursor[3];  // next alive-list tile of level i
-    unsigned long long out_len[3];   // survivors appended by level i's scan
     unsigned int next_min[3];        // smallest residual degree above level i
     unsigned int nonempty[3];        // some vertex was claimed at level i
     unsigned int err;                // KC_ERR_* raised on the device
@@ -83,7 +86,8 @@ struct PeelCtl {
     unsigned int level_indices;      // level indices processed
     unsigned int levels;             // non-empty levels
     unsigned int kmax;               // largest level with a claim
-    unsigned int pad;
+    unsigned int zeros;              // degree-0 vertices (level 0)
+    PeelDone done[3];
     PeelQueue q[3][PEEL_MAX_QUEUES]; // shared spill queues of level i (slot i % 3)
 };
 
@@ -155,7 +159,8 @@ struct Graph {
 
     // decomposition work buffers (allocated on first use, kept for reuse)
     uint32_t *bitmap = nullptr;       // [ceil(n/32)]  claimed / active flags
-    uint32_t *alive = nullptr;        // [2n]          alive lists (ping-pong by level)
+    uint32_t *alive = nullptr;        // alive lists, one pair per CTA of the peel (ping-pong by level)
+    uint64_t alive_cap = 0;           // entries of it
     unsigned long long *gq = nullptr; // spill queues of work items (sentinel = ~0)
     unsigned long long gq_cap = 0;    // capacity of each of the 3 x gq_nq queues
     unsigned gq_nq = 0;

@@ -6,11 +6,12 @@
 //
 // State per vertex: deg[v] (residual degree; equals the core number when the
 // kernel returns) and one bit in `claimed` (v has been peeled).  Per level L:
-//   * scan: CTA b takes tiles b, b + G, b + 2G, ... (threads x SCAN_U
-//     entries each) of the list of still-alive vertices, claims those with
-//     deg <= L (atomicOr on the claim bit decides a unique owner), appends
-//     the survivors to the next level's list and the claims to its queue
-//     (one reservation per warp) and records min(deg) of the survivors;
+//   * scan: every CTA owns the vertices of a fixed set of 32-vertex groups
+//     (see owned_group) and scans the list of those still alive: it claims the ones with deg <= L (atomicOr on the claim bit
+//     decides between it and a relaxing CTA), keeps the survivors as its next
+//     list and records their min(deg).  No CTA waits for another's list, and a
+//     list of at most LIST_CAP entries lives in shared memory, so a late
+//     level's scan is one gather of residual degrees;
 //   * process: balanced rounds spread the row entries of the queued items
 //     (up to round_e of them) over all threads of the CTA; rows above CHUNK
 //     entries are split into chunk items that any CTA may take, and the
@@ -26,9 +27,15 @@
 //   * level skipping: the next level is the smallest residual degree seen,
 //     not L+1, so empty levels cost nothing.
 // Work accounting instead of a grid barrier: every level has a counter of
-// outstanding credits (one per CTA until it finds no scan tile left and its
-// queue drained, plus every item put on the global queue).  A level ends when
-// the counter is zero.  All waits are bounded by a wall-clock limit and report
+// outstanding credits (one per CTA until its list is scanned and its queue
+// drained, plus every item put on the global queue).  A level ends when the
+// counter is zero; the CTA that brought it there announces the next level.
+// Against one alive list shared by all CTAs (a reservation per warp on one
+// counter, rewritten every level) and waits on the credit count itself:
+// Erdos-Renyi 65,536 / 1,048,576 0.325 -> 0.264 ms, R-MAT 18 2.94 -> 2.00,
+// R-MAT 22 6.87 -> 5.60, R-MAT 25 with a planted core 24.3 -> 22.3.  What bounds
+// it is the dependent steps of a level (scan, rounds, end) and, where a dense
+// core collapses, the rate of the L2's atomics.  All waits are bounded by a wall-clock limit and report
 // KC_ERR_TIMEOUT instead of hanging.
 #include <algorithm>
 #include <cstddef>
@@ -56,7 +63,15 @@ constexpr unsigned MIN_CHUNK = 256;   // smallest row chunk (sizes the shared qu
 constexpr unsigned long long SENT = ~0ull;
 constexpr unsigned int NO_LEVEL = 0xffffffffu;
 
-enum : int { M_SCAN = 1, M_PROC = 2, M_STEAL = 3, M_SPIN = 4, M_DONE = 5, M_EXIT = 6 };
+// The j-th 32-vertex group of CTA b: one of groups jG .. jG + G - 1, turned by
+// an odd number of places from one j to the next.  (Without the turn a CTA's
+// groups share their low bits when G is a multiple of 16, and on R-MAT graphs
+// those bits decide the degrees: R-MAT 25 took 28.5 ms instead of 23.0.)
+__device__ __forceinline__ unsigned long long owned_group(unsigned long long j, unsigned b, unsigned G) {
+    return j * G + (b + j * 97) % G;
+}
+
+enum : int { M_SCAN = 1, M_PROC = 2, M_STEAL = 3, M_DONE = 5, M_EXIT = 6 };
 
 struct PeelArgs {
     const int64_t *rowptr;
@@ -64,7 +79,8 @@ struct PeelArgs {
     uint32_t n;
     uint32_t *deg;
     uint32_t *claimed;
-    uint32_t *alive;  // two lists of n entries
+    uint32_t *alive;  // two lists of own_cap entries per CTA
+    uint64_t own_cap; // most vertices a CTA owns (a multiple of 32, below 2^32)
     unsigned long long *gq;      // 3 level slots x nq queues of gq_cap items
     unsigned long long gq_cap;
     PeelCtl *ctl;
@@ -83,16 +99,13 @@ struct PeelArgs {
 
 // Initialisation and level 0 in one streaming pass: residual degrees from the
 // row offsets; degree-0 vertices are peeled at level 0 (their claim bits are
-// written whole, one warp ballot per 32-vertex word); every other vertex is
-// appended to the alive list that level index 1 scans, and the smallest
-// degree among them becomes level index 1's level.
+// written whole, one warp ballot per 32-vertex word); the smallest degree
+// among the others becomes level index 1's level, whose scan takes the
+// vertices straight from the degrees.
 __global__ void peel_init(const int64_t *__restrict__ rowptr, uint32_t n, uint32_t *deg, uint32_t *claimed,
-                          uint32_t *alive1, PeelCtl *ctl, unsigned int grid) {
-    __shared__ unsigned int wcnt[32];
-    __shared__ unsigned long long base_sh;
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    unsigned dmin = 0xffffffffu;
-    bool any_zero = false;
+                          PeelCtl *ctl) {
+    const unsigned lane = threadIdx.x & 31;
+    unsigned dmin = 0xffffffffu, zeros = 0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t b0 = (uint64_t)blockIdx.x * blockDim.x; b0 < n; b0 += stride) {
         const uint64_t v = b0 + threadIdx.x;  // b0 is a multiple of 32: a warp covers one bitmap word
@@ -104,49 +117,35 @@ __global__ void peel_init(const int64_t *__restrict__ rowptr, uint32_t n, uint32
         }
         const unsigned zero = __ballot_sync(KC_FULL_MASK, inr && d == 0);
         if (lane == 0 && v < n) claimed[v >> 5] = zero;
-        any_zero |= zero != 0u;
-        const bool keep = inr && d != 0;
-        if (keep) dmin = min(dmin, d);
-        const unsigned kb = __ballot_sync(KC_FULL_MASK, keep);
-        if (lane == 0) wcnt[warp] = __popc(kb);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned tot = 0;
-            for (unsigned w = 0; w < nw; w++) {
-                unsigned c = wcnt[w];
-                wcnt[w] = tot;
-                tot += c;
-            }
-            base_sh = tot ? atomicAdd(&ctl->out_len[0], (unsigned long long)tot) : 0ull;
-        }
-        __syncthreads();
-        if (keep) alive1[base_sh + wcnt[warp] + __popc(kb & ((1u << lane) - 1u))] = (uint32_t)v;
-        __syncthreads();
+        zeros += __popc(zero);
+        if (d != 0) dmin = min(dmin, d);
     }
     dmin = __reduce_min_sync(KC_FULL_MASK, dmin);
     if (lane == 0 && dmin != 0xffffffffu) atomicMin(&ctl->next_min[0], dmin);
-    if (__any_sync(KC_FULL_MASK, any_zero) && lane == 0) atomicExch(&ctl->nonempty[0], 1u);
+    if (lane == 0 && zeros) atomicAdd(&ctl->zeros, zeros);
 }
 
-// Resets the control block before peel_init runs.
+// Resets the control block before peel_init runs (one thread per queue).
 __global__ void peel_ctl_reset(PeelCtl *ctl, unsigned int grid) {
-    for (int i = 0; i < 3; i++) {
-        ctl->pending[i] = grid;
-        ctl->scan_cursor[i] = 0;
-        ctl->out_len[i] = 0;
-        ctl->next_min[i] = NO_LEVEL;
-        ctl->nonempty[i] = 0;
+    const unsigned t = threadIdx.x;
+    if (t < 3 * PEEL_MAX_QUEUES) {
+        ctl->q[t / PEEL_MAX_QUEUES][t % PEEL_MAX_QUEUES].head = 0;
+        ctl->q[t / PEEL_MAX_QUEUES][t % PEEL_MAX_QUEUES].tail = 0;
     }
-    for (int sl = 0; sl < 3; sl++)
-        for (int i = 0; i < PEEL_MAX_QUEUES; i++) {
-            ctl->q[sl][i].head = 0;
-            ctl->q[sl][i].tail = 0;
-        }
-    ctl->err = 0;
-    ctl->err_info = 0;
-    ctl->level_indices = 0;
-    ctl->levels = 0;
-    ctl->kmax = 0;
+    if (t < 3) {
+        ctl->done[t].word = 0;
+        ctl->pending[t] = grid;
+        ctl->next_min[t] = NO_LEVEL;
+        ctl->nonempty[t] = 0;
+    }
+    if (t == 0) {
+        ctl->zeros = 0;
+        ctl->err = 0;
+        ctl->err_info = 0;
+        ctl->level_indices = 0;
+        ctl->levels = 0;
+        ctl->kmax = 0;
+    }
 }
 
 // Degree-0 vertices get core 1 in GPP mode (gppeel.cu:35-39: its first
@@ -172,20 +171,22 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
     constexpr int PEEL_THREADS = NT;
     constexpr int PEEL_WARPS = NT / 32;
     constexpr unsigned TILE = NT * SCAN_U;
+    constexpr unsigned LIST_CAP = TILE < 2048 ? TILE : 2048;  // scanned in one tile
     __shared__ unsigned long long q[QCAP];
     __shared__ unsigned int q_head, q_tail;
     __shared__ unsigned int q_res;  // scan: queue slots reserved so far in this tile
     __shared__ int mode;
     __shared__ unsigned int b_base, b_per_warp, b_take;
-    __shared__ unsigned long long tile_base, scan_len;
-    __shared__ unsigned int scan_done;
+    __shared__ unsigned int tile_base, next_tile;
+    __shared__ unsigned int list_len, kept;  // this CTA's list, survivors of it so far
+    __shared__ uint32_t list_sh[LIST_CAP];         // the list once it is this short
+    __shared__ unsigned int list_in_sh, scan_done;
     __shared__ unsigned long long credit;
     __shared__ unsigned int min_sh, claimed_any;
     __shared__ unsigned long long res_base, res_mask;  // reserved queue slots still expected
     __shared__ unsigned int steal_cnt, probe, claims_sh, spill_rr;
-    __shared__ unsigned int level_sh, li_sh;
+    __shared__ unsigned int level_sh, li_sh, next_level;
     __shared__ unsigned long long wait_t0;
-    __shared__ unsigned long long next_tile;
     __shared__ unsigned int withheld;
     __shared__ unsigned int rounds_sh;
     __shared__ unsigned long long mode_ns[4], mode_t0;  // trace: time per mode in this level
@@ -204,7 +205,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
         q_head = q_tail = 0;
         level_sh = ld_acquire(&ctl->next_min[0]);
         li_sh = 1;
-        scan_len = ld_relaxed64(&ctl->out_len[0]);
+        list_len = (unsigned)A.own_cap;  // owned_group() beyond the last vertex is skipped by the scan
+        kept = 0;
+        list_in_sh = 0;
         probe = blockIdx.x;
         spill_rr = blockIdx.x;
         res_mask = 0;
@@ -215,17 +218,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
     if (level_sh == NO_LEVEL) {  // every vertex had degree 0
         if (blockIdx.x == 0 && tid == 0) {
             ctl->level_indices = 1;
-            ctl->levels = ld_relaxed(&ctl->nonempty[0]) ? 1u : 0u;
+            ctl->levels = ld_relaxed(&ctl->zeros) ? 1u : 0u;
         }
         return;
     }
     if (blockIdx.x == 0 && tid == 0) {
-        if (ld_relaxed(&ctl->nonempty[0])) ctl->levels = 1;
+        if (ld_relaxed(&ctl->zeros)) ctl->levels = 1;
         if (A.trace && A.trace_cap) {
             A.trace[0].t_start_ns = global_ns();
             A.trace[0].level = 0;
             A.trace[0].scan_len = n;
-            A.trace[0].claimed = n - (unsigned)scan_len;
+            A.trace[0].claimed = ld_relaxed(&ctl->zeros);
         }
     }
 
@@ -233,14 +236,12 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
         const unsigned li = li_sh;
         const unsigned L = level_sh;
         const unsigned s = li % 3;
-        const uint32_t *src = A.alive + (size_t)(li & 1) * n;
-        uint32_t *dst = A.alive + (size_t)((li + 1) & 1) * n;
+        const uint32_t *src = A.alive + ((size_t)(li & 1) * G + blockIdx.x) * A.own_cap;
+        uint32_t *dst = A.alive + ((size_t)((li + 1) & 1) * G + blockIdx.x) * A.own_cap;
         if (tid == 0) {
             if (blockIdx.x == 0) {
                 unsigned s1 = (li + 1) % 3;
                 ctl->pending[s1] = G;
-                ctl->scan_cursor[s1] = 0;
-                ctl->out_len[s1] = 0;
                 ctl->next_min[s1] = NO_LEVEL;
                 ctl->nonempty[s1] = 0;
                 for (unsigned i = 0; i < A.nq; i++) {
@@ -252,11 +253,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
             if (A.trace && blockIdx.x == 0 && li < A.trace_cap) {
                 A.trace[li].t_start_ns = global_ns();
                 A.trace[li].level = L;
-                A.trace[li].scan_len = (unsigned)scan_len;
             }
+            if (A.trace && li < A.trace_cap) atomicAdd(&A.trace[li].scan_len, list_len);
             claims_sh = 0;
-            next_tile = blockIdx.x;  // tiles blockIdx.x, +G, +2G, ... of the alive list
-            scan_done = (scan_len == 0);
+            next_tile = 0;
+            scan_done = (list_len == 0);
             credit = 1;  // this CTA's token for the level
             min_sh = NO_LEVEL;
             claimed_any = 0;
@@ -265,10 +266,56 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
             if (A.trace) {
                 mode_ns[0] = mode_ns[1] = mode_ns[2] = mode_ns[3] = 0;
                 mode_t0 = global_ns();
-                prev_mode = M_SPIN;
+                prev_mode = M_SCAN;
             }
         }
         __syncthreads();
+
+        // A list of at most one entry per thread is scanned right here.  Late
+        // levels mostly claim nothing in most CTAs: their whole scan is one
+        // gather of residual degrees, a minimum and a barrier, and the list
+        // stays as it is.
+        if (list_in_sh && list_len <= NT) {
+            const bool in = tid < list_len;
+            const uint32_t v = in ? list_sh[tid] : 0u;
+            const unsigned d = in ? __ldcg(&A.deg[v]) : NO_LEVEL;
+            const bool want = in && (int)d <= (int)L;
+            const unsigned dmin = __reduce_min_sync(KC_FULL_MASK, want ? NO_LEVEL : d);
+            if (lane == 0 && dmin != NO_LEVEL) atomicMin(&min_sh, dmin);
+            if (!__syncthreads_or(want)) {
+                if (tid == 0) {
+                    kept = list_len;
+                    scan_done = 1;
+                }
+            } else {
+                // the claim and the row offsets it needs travel together
+                unsigned old = ~0u;
+                int64_t r0 = 0, r1 = 0;
+                if (want) {
+                    old = atomicOr(&A.claimed[v >> 5], 1u << (v & 31));
+                    r0 = A.rowptr[v];
+                    r1 = A.rowptr[v + 1];
+                }
+                const bool keep = in && !want, take = want && !(old & (1u << (v & 31)));
+                const unsigned kb = __ballot_sync(KC_FULL_MASK, keep), cb = __ballot_sync(KC_FULL_MASK, take);
+                unsigned kbase = 0, qb = 0;
+                if (lane == 0 && kb) kbase = atomicAdd(&kept, (unsigned)__popc(kb));
+                if (lane == 0 && cb) {
+                    qb = atomicAdd(&q_tail, __popc(cb));  // the queue is empty: room for all
+                    claimed_any = 1;
+                    if (A.trace) atomicAdd(&claims_sh, __popc(cb));
+                }
+                kbase = __shfl_sync(KC_FULL_MASK, kbase, 0);
+                qb = __shfl_sync(KC_FULL_MASK, qb, 0);
+                const unsigned lt = (1u << lane) - 1u;
+                if (keep) list_sh[kbase + __popc(kb & lt)] = v;
+                if (take)
+                    q[(qb + __popc(cb & lt)) % QCAP] =
+                        range_fits(r0, r1) ? range_item(r0, (uint32_t)(r1 - r0)) : (unsigned long long)v << 32;
+                if (tid == 0) scan_done = 1;
+            }
+            __syncthreads();
+        }
 
         for (;;) {  // work loop of one level
             if (tid == 0) {
@@ -279,10 +326,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                 // reading the flag every step would put one more round trip
                 // on the path of every scan tile and processing round
                 if (!scan_done && qsize < SCAN_BELOW) {
-                    unsigned long long t = next_tile * TILE;
-                    if (t < scan_len) {
-                        tile_base = t;
-                        next_tile += G;
+                    if (next_tile < list_len) {
+                        tile_base = next_tile;
+                        next_tile += TILE;
                         q_res = q_tail;
                         md = M_SCAN;
                     } else {
@@ -306,10 +352,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                     md = M_PROC;
                     rounds_sh++;
                 }
-                if (!md && ld_relaxed(&ctl->err) != 0) md = M_EXIT;
                 if (!md) {
                     // idle: hand back the credits held, after publishing this
-                    // CTA's level minimum and claim flag
+                    // CTA's level minimum and claim flag.  The CTA whose
+                    // credits bring the count to zero ends the level: it alone
+                    // reads the level's results and announces the next level.
                     if (credit > 0) {
                         if (A.trace && li < A.trace_cap) {
                             if (claims_sh) atomicAdd(&A.trace[li].claimed, claims_sh);
@@ -322,7 +369,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                             ctl->nonempty[s] = 1u;
                             atomicMax(&ctl->kmax, L);
                         }
-                        __threadfence();
+                        fence_acq_rel();
                         unsigned long long give = credit;
                         if (A.withhold && blockIdx.x == 0 && li == 1 && !withheld) {
                             // the level's count can no longer reach zero: every
@@ -330,59 +377,92 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                             give -= 1;
                             withheld = 1;
                         }
-                        atomicAdd(&ctl->pending[s], (unsigned long long)(0ull - give));
+                        const unsigned long long had = atomicAdd(&ctl->pending[s], (unsigned long long)(0ull - give));
                         credit = 0;
-                    }
-                    // Shared queues: a CTA reserves up to steal_max slots with one
-                    // atomicAdd on the queue head (never fails) and takes the
-                    // items as producers fill them.  Slots still empty when the
-                    // level's credit count reaches zero will never be filled
-                    // (producers push only while holding credit) and are dropped.
-                    md = M_SPIN;
-                    if (res_mask == 0) {
-                        for (unsigned k = 0; k < A.nq; k++) {
-                            const unsigned qi = (probe + k) % A.nq;
-                            unsigned long long h = ld_relaxed64(&ctl->q[s][qi].head);
-                            unsigned long long t = ld_relaxed64(&ctl->q[s][qi].tail);
-                            if (t > A.gq_cap) t = A.gq_cap;  // an overflow was flagged; never read past the end
-                            if (h >= t) continue;
-                            unsigned long long want = (t - h + 3) / 4;
-                            if (want > A.steal_max) want = A.steal_max;
-                            unsigned long long r = atomicAdd(&ctl->q[s][qi].head, want);
-                            if (r < A.gq_cap) {
-                                if (r + want > A.gq_cap) want = A.gq_cap - r;
-                                res_base = ((unsigned long long)s * A.nq + qi) * A.gq_cap + r;
-                                res_mask = want >= 64 ? ~0ull : ((1ull << want) - 1);
-                                if (A.trace && li < A.trace_cap) {
-                                    atomicAdd(&A.trace[li].steals, 1u);
-                                    atomicMax(&A.trace[li].max_steal, (unsigned)want);
-                                }
+                        if (had == give && give) {
+                            fence_acq_rel();
+                            unsigned nxt = ld_relaxed(&ctl->next_min[s]);
+                            const unsigned any = ld_relaxed(&ctl->nonempty[s]);
+                            if (nxt != NO_LEVEL && li + 1 >= A.max_level_indices) {
+                                set_err(ctl, KC_ERR_CAPACITY, 5);
+                                nxt = NO_LEVEL;
                             }
-                            probe = qi;
+                            st_relaxed64(&ctl->done[s].word, ((unsigned long long)li << 32) | nxt);
+                            atomicMax(&ctl->level_indices, li + 1);
+                            if (any) atomicAdd(&ctl->levels, 1u);
+                        }
+                    }
+                    // Wait for work or for the level's end.  Shared queues: a
+                    // CTA reserves up to steal_max slots with one atomicAdd on
+                    // the queue head (never fails) and takes the items as
+                    // producers fill them.  Slots still empty when the level is
+                    // over will never be filled (producers push only while
+                    // holding credit) and are dropped.  The end is read from a
+                    // word written once per level, on a line of its own: polls
+                    // of the credit count would delay the credits still coming,
+                    // and polls of the queues delay their producers, so those
+                    // are read one time in four (R-MAT 22: every 100 ns, all of
+                    // them, 5.88 ms; every 200 ns and one in four 5.60 ms).
+                    if (A.trace) {
+                        const unsigned long long now = global_ns();
+                        mode_ns[prev_mode == M_SCAN ? 0 : prev_mode == M_PROC ? 1 : 2] += now - mode_t0;
+                        mode_t0 = now;
+                        prev_mode = M_DONE;
+                    }
+                    for (unsigned polls = 0;;) {
+                        const unsigned err = ld_relaxed(&ctl->err);
+                        const unsigned long long done = ld_acquire64(&ctl->done[s].word);
+                        if (res_mask == 0 && (polls++ & 3u) == 0) {
+                            for (unsigned k = 0; k < A.nq; k++) {
+                                const unsigned qi = (probe + k) % A.nq;
+                                unsigned long long h = ld_relaxed64(&ctl->q[s][qi].head);
+                                unsigned long long t = ld_relaxed64(&ctl->q[s][qi].tail);
+                                if (t > A.gq_cap) t = A.gq_cap;  // an overflow was flagged; never read past the end
+                                if (h >= t) continue;
+                                unsigned long long want = (t - h + 3) / 4;
+                                if (want > A.steal_max) want = A.steal_max;
+                                unsigned long long r = atomicAdd(&ctl->q[s][qi].head, want);
+                                if (r < A.gq_cap) {
+                                    if (r + want > A.gq_cap) want = A.gq_cap - r;
+                                    res_base = ((unsigned long long)s * A.nq + qi) * A.gq_cap + r;
+                                    res_mask = want >= 64 ? ~0ull : ((1ull << want) - 1);
+                                    if (A.trace && li < A.trace_cap) {
+                                        atomicAdd(&A.trace[li].steals, 1u);
+                                        atomicMax(&A.trace[li].max_steal, (unsigned)want);
+                                    }
+                                }
+                                probe = qi;
+                                break;
+                            }
+                        }
+                        if (err != 0) {
+                            md = M_EXIT;
                             break;
                         }
-                    }
-                    if (res_mask != 0) {
-                        const unsigned j0 = __ffsll((long long)res_mask) - 1;
-                        if (ld_relaxed64(&A.gq[res_base + j0]) != SENT) {
-                            md = M_STEAL;
-                            wait_t0 = 0;
-                        } else if (A.trace && li < A.trace_cap) {
-                            atomicAdd(&A.trace[li].steal_fail, 1u);
-                        }
-                    }
-                    if (md == M_SPIN) {
-                        if (ld_acquire64(&ctl->pending[s]) == 0ull) {
-                            res_mask = 0;  // the level is over: nothing more will arrive
-                            md = M_DONE;
-                        } else {
-                            unsigned long long now = global_ns();
-                            if (wait_t0 == 0) wait_t0 = now;
-                            else if (now - wait_t0 > A.timeout_ns) {
-                                set_err(ctl, KC_ERR_TIMEOUT, 1);
-                                md = M_EXIT;
+                        if (res_mask != 0) {
+                            const unsigned j0 = __ffsll((long long)res_mask) - 1;
+                            if (ld_relaxed64(&A.gq[res_base + j0]) != SENT) {
+                                md = M_STEAL;
+                                wait_t0 = 0;
+                                break;
                             }
+                            if (A.trace && li < A.trace_cap) atomicAdd(&A.trace[li].steal_fail, 1u);
                         }
+                        if ((done >> 32) == li) {
+                            res_mask = 0;  // the level is over: nothing more will arrive
+                            next_level = (unsigned)done;
+                            md = M_DONE;
+                            break;
+                        }
+                        const unsigned long long now = global_ns();
+                        if (wait_t0 == 0) {
+                            wait_t0 = now;
+                        } else if (now - wait_t0 > A.timeout_ns) {
+                            set_err(ctl, KC_ERR_TIMEOUT, 1);
+                            md = M_EXIT;
+                            break;
+                        }
+                        __nanosleep(200);
                     }
                 }
                 mode = md;
@@ -398,12 +478,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
             __syncthreads();
             const int md = mode;
             if (md == M_DONE || md == M_EXIT) break;
-
-            if (md == M_SPIN) {
-                if (tid == 0) __nanosleep(100);
-                __syncthreads();
-                continue;
-            }
 
             if (md == M_STEAL) {
                 // take every filled slot of the reservation into the CTA queue
@@ -430,15 +504,22 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
             }
 
             if (md == M_SCAN) {
-                // ---- scan one tile (SCAN_U entries per thread) of the alive list
+                // ---- scan one tile (SCAN_U entries per thread) of this CTA's list
                 uint32_t v[SCAN_U];
                 unsigned d[SCAN_U];
                 bool inr[SCAN_U], keep[SCAN_U];
+                const bool in_sh = list_in_sh != 0, to_sh = list_len <= LIST_CAP;
 #pragma unroll
                 for (int k = 0; k < SCAN_U; k++) {
-                    const unsigned long long pos = tile_base + (unsigned)k * PEEL_THREADS + tid;
-                    inr[k] = pos < scan_len;
-                    v[k] = inr[k] ? src[pos] : 0u;
+                    const unsigned pos = tile_base + (unsigned)k * PEEL_THREADS + tid;
+                    inr[k] = pos < list_len;
+                    if (li == 1) {  // no list yet: the owned groups themselves
+                        const unsigned long long own = owned_group(pos >> 5, blockIdx.x, G) * 32 + (pos & 31);
+                        inr[k] = inr[k] && own < n;
+                        v[k] = (uint32_t)own;
+                    } else {
+                        v[k] = inr[k] ? (in_sh ? list_sh[pos % LIST_CAP] : src[pos]) : 0u;
+                    }
                 }
                 // The residual degree alone sorts the entries: a vertex peeled
                 // at an earlier level holds its level (< L); one peeled at this
@@ -449,6 +530,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                 // at an earlier level) already had.
 #pragma unroll
                 for (int k = 0; k < SCAN_U; k++) d[k] = inr[k] ? __ldcg(&A.deg[v[k]]) : 0u;
+                if (in_sh) __syncthreads();  // every entry has been read: survivors may overwrite them
                 unsigned dkeep = NO_LEVEL;
                 // claims: lanes whose vertices share a bitmap word set their
                 // bits with one atomicOr by the lowest such lane; all the
@@ -459,23 +541,26 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                 unsigned kcnt = 0;
 #pragma unroll
                 for (int k = 0; k < SCAN_U; k++) {
+                    if (li == 1) inr[k] = inr[k] && d[k] != 0;  // peeled by peel_init
                     keep[k] = inr[k] && (int)d[k] > (int)L;
                     if (keep[k]) dkeep = min(dkeep, d[k]);
                     const bool want = inr[k] && !keep[k];
-                    const unsigned word = want ? (v[k] >> 5) : 0xffffffffu;
-                    const unsigned bit = want ? (1u << (v[k] & 31)) : 0u;
-                    const unsigned peers = __match_any_sync(KC_FULL_MASK, word);
-                    const unsigned bits = __reduce_or_sync(peers, bit);
-                    leader[k] = __ffs(peers) - 1;
                     oldw[k] = 0;
-                    if (want && (int)lane == leader[k]) oldw[k] = atomicOr(&A.claimed[word], bits);
+                    leader[k] = 0;
+                    if (__any_sync(KC_FULL_MASK, want)) {
+                        const unsigned word = want ? (v[k] >> 5) : 0xffffffffu;
+                        const unsigned bit = want ? (1u << (v[k] & 31)) : 0u;
+                        const unsigned peers = __match_any_sync(KC_FULL_MASK, word);
+                        const unsigned bits = __reduce_or_sync(peers, bit);
+                        leader[k] = __ffs(peers) - 1;
+                        if (want && (int)lane == leader[k]) oldw[k] = atomicOr(&A.claimed[word], bits);
+                    }
                     kb[k] = __ballot_sync(KC_FULL_MASK, keep[k]);
                     kcnt += __popc(kb[k]);
                 }
-                // survivors: each warp reserves its run of the next alive list
-                // with one atomicAdd, in flight with the claim atomics
-                unsigned long long wbase = 0;
-                if (lane == 0 && kcnt) wbase = atomicAdd(&ctl->out_len[s], (unsigned long long)kcnt);
+                // survivors: each warp reserves its run of the CTA's next list
+                unsigned wbase = 0;
+                if (lane == 0 && kcnt) wbase = atomicAdd(&kept, kcnt);
                 dkeep = __reduce_min_sync(KC_FULL_MASK, dkeep);
                 if (lane == 0 && dkeep != NO_LEVEL) atomicMin(&min_sh, dkeep);
                 unsigned cb[SCAN_U];
@@ -503,7 +588,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                 unsigned ko = 0, co = 0;
 #pragma unroll
                 for (int k = 0; k < SCAN_U; k++) {
-                    if (keep[k]) dst[wbase + ko + __popc(kb[k] & lt)] = v[k];
+                    if (keep[k]) {
+                        const unsigned at = wbase + ko + __popc(kb[k] & lt);
+                        if (to_sh) list_sh[at] = v[k];
+                        else dst[at] = v[k];
+                    }
                     if (cb[k] & (1u << lane)) q[(qb + co + __popc(cb[k] & lt)) % QCAP] = ((unsigned long long)v[k] << 32);
                     ko += __popc(kb[k]);
                     co += __popc(cb[k]);
@@ -631,6 +720,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                 unsigned local_min = NO_LEVEL;
                 unsigned wclaims = 0;
                 for (unsigned base = 0; base < total; base += SPAN * PEEL_U) {
+                    // steps with entries left (small rounds have one)
+                    const unsigned steps = (total - base + SPAN - 1) / SPAN;
                     uint32_t u[PEEL_U];
                     unsigned a[PEEL_U];
                     bool live[PEEL_U];
@@ -640,6 +731,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                         int64_t rj;
                         unsigned oj;
                         live[k] = e < total;
+                        u[k] = 0;
+                        if (k >= (int)steps) continue;
                         if constexpr (BAL) {
                             // owner item: the last j with bal_off[j] <= e
                             unsigned lo = 0, hi2 = bal_n;
@@ -705,7 +798,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                     for (int k = 0; k < PEEL_U; k++) {
                         oldc[k] = ~0u;
                         cr0[k] = cr1[k] = 0;
-                        if (live[k]) {
+                        if (k < (int)steps && live[k]) {
                             const unsigned nv = a[k] - cnt[k];
                             if ((int)a[k] <= (int)L) {
                                 atomicAdd(&A.deg[u[k]], cnt[k]);
@@ -721,6 +814,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                     }
 #pragma unroll
                     for (int k = 0; k < PEEL_U; k++) {
+                        if (k >= (int)steps) break;
                         const bool push = !(oldc[k] & (1u << (u[k] & 31)));
                         unsigned pb = __ballot_sync(KC_FULL_MASK, push);
                         wclaims += __popc(pb);
@@ -787,20 +881,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
         if (tid == 0) {
             unsigned nxt = NO_LEVEL;
             if (mode == M_DONE) {
-                // pending reached zero (read with acquire) after every CTA's
-                // last update of this slot: both values are final and are
-                // fetched together
-                __threadfence();
-                nxt = ld_relaxed(&ctl->next_min[s]);
-                scan_len = ld_relaxed64(&ctl->out_len[s]);
-                if (blockIdx.x == 0) {
-                    ctl->level_indices = li + 1;
-                    if (ld_relaxed(&ctl->nonempty[s])) ctl->levels += 1;
-                }
-                if (nxt != NO_LEVEL && li + 1 >= A.max_level_indices) {
-                    set_err(ctl, KC_ERR_CAPACITY, 5);
-                    nxt = NO_LEVEL;
-                }
+                nxt = next_level;
+                list_in_sh = list_len <= LIST_CAP;
+                list_len = kept;
+                kept = 0;
             }
             level_sh = nxt;
             li_sh = li + 1;
@@ -811,11 +895,20 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
 }
 
 // ------------------------------------------------------------ host -------
-static int ensure_peel_buffers(Graph *g) {
+// The most vertices one of `grid` CTAs owns (whole groups of 32).
+static uint64_t own_cap(uint64_t n, uint64_t grid) { return ((n + 31) / 32 + grid - 1) / grid * 32; }
+
+static int ensure_peel_buffers(Graph *g, uint64_t grid) {
     const uint64_t n = g->n;
     if (!g->core) KC_TRY(dalloc(&g->core, n + 1, "core"));
     if (!g->bitmap) KC_TRY(dalloc(&g->bitmap, (n + 31) / 32 + 1, "claim bitmap"));
-    if (!g->alive) KC_TRY(dalloc(&g->alive, 2 * n + 2, "alive lists"));
+    const uint64_t alive = 2 * grid * own_cap(n, grid);
+    if (!g->alive || g->alive_cap < alive) {
+        dfree(g->alive);
+        g->alive = nullptr;
+        KC_TRY(dalloc(&g->alive, alive, "alive lists"));
+        g->alive_cap = alive;
+    }
     const unsigned nq = (unsigned)g->tune.peel_queues;
     const unsigned long long items = n + g->nnz / MIN_CHUNK + 64;
     if (!g->gq || g->gq_nq != nq || g->gq_items < items) {
@@ -878,7 +971,6 @@ static int peel_grid(const void *kern, int threads, int sm_count, int ctas_per_s
 static unsigned nq_of(const Graph *g) { return g->gq_nq; }
 
 int peel_run(Graph *g, cudaStream_t s, bool gpp_zero_to_one_flag, kc_stats *st) {
-    KC_TRY(ensure_peel_buffers(g));
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, g->device);
     if (!coop) return fail(KC_ERR_UNSUPPORTED, "device lacks cooperative launch");
@@ -886,6 +978,7 @@ int peel_run(Graph *g, cudaStream_t s, bool gpp_zero_to_one_flag, kc_stats *st) 
     int threads = 0;
     const void *kern = peel_variant(g->tune, &threads);
     KC_TRY(peel_grid(kern, threads, g->sm_count, g->tune.peel_ctas_per_sm, &grid));
+    KC_TRY(ensure_peel_buffers(g, (uint64_t)grid));
     if (!g->gq_clean) {
         KC_CUDA(cudaMemsetAsync(g->gq, 0xff, 3 * g->gq_cap * g->gq_nq * sizeof(unsigned long long), s));
         g->gq_clean = true;
@@ -903,6 +996,7 @@ int peel_run(Graph *g, cudaStream_t s, bool gpp_zero_to_one_flag, kc_stats *st) 
     A.deg = g->core;
     A.claimed = g->bitmap;
     A.alive = g->alive;
+    A.own_cap = own_cap(g->n, (uint64_t)grid);
     A.gq = g->gq;
     A.gq_cap = g->gq_cap;
     A.ctl = g->peel_ctl;
@@ -922,8 +1016,8 @@ int peel_run(Graph *g, cudaStream_t s, bool gpp_zero_to_one_flag, kc_stats *st) 
     KC_CUDA(cudaEventRecord(g->ev0, s));
     if (A.trace) KC_CUDA(cudaMemsetAsync(g->trace, 0, sizeof(PeelTrace) * g->trace_cap, s));
     const int ig = std::max(1, std::min<int>(g->sm_count * 8, (int)((g->n + 255) / 256)));
-    peel_ctl_reset<<<1, 1, 0, s>>>(g->peel_ctl, (unsigned)grid);
-    peel_init<<<ig, 256, 0, s>>>(g->rowptr, g->n, g->core, g->bitmap, g->alive + g->n, g->peel_ctl, (unsigned)grid);
+    peel_ctl_reset<<<1, 3 * PEEL_MAX_QUEUES, 0, s>>>(g->peel_ctl, (unsigned)grid);
+    peel_init<<<ig, 256, 0, s>>>(g->rowptr, g->n, g->core, g->bitmap, g->peel_ctl);
     void *args[] = {&A};
     KC_CUDA(cudaEventRecord(g->evk0, s));
     KC_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(threads), args, 0, s));
