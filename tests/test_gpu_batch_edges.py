@@ -73,3 +73,25 @@ def test_noalloc_edges(part):
     assert np.array_equal(out.download(np.uint32, g.n), oracle.bz(*g.csr())[0])
     out.free()
     g.free()
+
+
+def test_batch_plan_over_empty_graphs_and_tiles():
+    """Segments of 0, 1 and up to 9,000 vertices (tiles of 4,096 vertices and
+    entries end inside, at and between graphs), with edgeless ones first and
+    last; then one vertex moved to its neighbour's segment is refused."""
+    rng = np.random.default_rng(5)
+    sizes = [0, 1, 0, 0, 3, 4095, 1, 4096, 0, 2, 9000, 31, 0, 5000, 64, 1, 0]
+    parts = [random_graph(n, 3 * n, n) if n > 2 else (n, np.zeros(0, np.uint32), np.zeros(0, np.uint32)) for n in sizes]
+    g, vbase = pack(parts)
+    want = oracle.bz(*g.csr())[0]
+    b = pg.Batch(g, vbase)
+    assert np.array_equal(b.decompose()[0], want)
+    b.free()
+    for i in (5, 7, 10, 13):  # the first vertex of a connected segment into the one before
+        moved = vbase.copy()
+        moved[i] += 1
+        for j in range(i - 1, 0, -1):
+            moved[j] = min(moved[j], moved[i])
+        with pytest.raises(pg.KCoreError):
+            pg.Batch(g, moved)
+    g.free()
