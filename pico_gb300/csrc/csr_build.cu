@@ -9,11 +9,12 @@
 //   3. scatter of both directions of every edge into its row,
 //   4. segmented row sort -- by neighbour id (dedup / sorted rows) or by the
 //      entry's position in the edge list (the row order MakeUGraph produces),
-//      with three size classes: <=32 entries (one warp, register bitonic),
-//      <=4096 (one CTA, shared-memory bitonic), larger (one CTA, stable LSD
-//      radix through a global staging buffer),
+//      with three size classes: <=32 entries (one warp, shuffle bitonic),
+//      <=4096 (one to eight warps, register bitonic), larger (one CTA, a column
+//      bitmap or a stable LSD radix through a global staging buffer),
 //   5. optional unique per row, rescan and compaction.
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "kc_device.cuh"
@@ -190,13 +191,12 @@ __global__ void scatter_edges(const uint32_t *__restrict__ src, const uint32_t *
 // ------------------------------------------------------ segmented sort ----
 // Rows are sorted by size class: up to 32 entries one warp per row (shuffle
 // bitonic network); 33..4096 entries padded to P = 2^k (k = 6..12) and sorted
-// SORT_PACK / P rows at a time per CTA in shared memory (one bitonic network,
-// so short rows share the barriers instead of occupying a CTA each); longer
-// rows one CTA per row with an LSD radix sort.
+// in registers, by one to eight warps a row; longer rows one CTA per row, with
+// a bitmap where repeated entries are dropped anyway and an LSD radix sort
+// elsewhere.
 constexpr uint32_t CLASS_A_MAX = 32;
 constexpr uint32_t CLASS_B_MAX = 4096;
 constexpr int SORT_BUCKETS = 9;  // 0: <= 32; 1..7: P = 64..4096; 8: > 4096
-constexpr uint32_t SORT_PACK = 1024;
 
 __device__ __forceinline__ int sort_bucket(int64_t len) {
     if (len < 2) return -1;
@@ -270,67 +270,227 @@ __global__ void sort_rows_warp(const int64_t *__restrict__ rowptr, const uint32_
     }
 }
 
-// Class B: rows of P/2 < len <= P entries (P = 2^LOGP, 64..4096), padded to
-// P with the largest key, SORT_PACK / P rows per CTA (one row for P > 1024).
-template <bool HAS_VAL, int LOGP>
-__global__ void __launch_bounds__(256) sort_rows_pack(const int64_t *__restrict__ rowptr,
-                                                      const uint32_t *__restrict__ rows, uint64_t nrows,
-                                                      uint32_t *key, uint32_t *val) {
-    constexpr uint32_t P = 1u << LOGP;
-    constexpr uint32_t E = P > SORT_PACK ? P : SORT_PACK;  // elements per CTA
-    constexpr uint32_t RPC = E / P;                          // rows per CTA
-    __shared__ uint32_t sk[E];
-    __shared__ uint32_t sv[HAS_VAL ? E : 1];
-    __shared__ int64_t rstart[RPC];
-    __shared__ uint32_t rlen[RPC];
-    for (uint64_t grp = blockIdx.x; grp * RPC < nrows; grp += gridDim.x) {
-        if (threadIdx.x < RPC) {
-            const uint64_t r = grp * RPC + threadIdx.x;
-            if (r < nrows) {
-                const uint32_t v = rows[r];
-                rstart[threadIdx.x] = rowptr[v];
-                rlen[threadIdx.x] = (uint32_t)(rowptr[v + 1] - rowptr[v]);
-            } else {
-                rstart[threadIdx.x] = 0;
-                rlen[threadIdx.x] = 0;
+// Class B: rows of P/2 < len <= P = 32 R W entries, padded to P with the
+// largest key, in the registers of W warps: a bitonic network in which lane l
+// of warp w holds entries (32 w + l) R + j, so that strides below R are
+// compares within a lane, strides below 32 R shuffles, and only the widest
+// strides of rows above 1,024 entries go through shared memory (1 and 3 steps
+// of 66 and 78).  A phase that sorts downwards on a lane runs upwards on
+// complemented keys.  Keys are loaded in any order and stored in row order
+// through shared memory.  What bounds it is the instructions of the compares;
+// the network in shared memory that it replaces paid two reads, two writes and
+// a barrier a step (R-MAT 22, 134 M entries, rows of 33..4,096: 2.66 ms, now
+// 0.77 ms).
+constexpr int SORT_THREADS = 256;
+
+template <bool HAS_VAL>
+__device__ __forceinline__ void sort_pair(uint32_t &ka, uint32_t &va, uint32_t &kb, uint32_t &vb, bool up) {
+    if (HAS_VAL) {
+        if ((kb < ka) == up && ka != kb) {
+            uint32_t t = ka;
+            ka = kb;
+            kb = t;
+            t = va;
+            va = vb;
+            vb = t;
+        }
+    } else {
+        const uint32_t lo = min(ka, kb), hi = max(ka, kb);
+        ka = up ? lo : hi;
+        kb = up ? hi : lo;
+    }
+}
+
+// The compares of one phase (entries at distance top, top / 2, .. 1, all within
+// a warp's 32 R entries).  up(j): whether entry j of a lane sorts upwards.
+template <bool HAS_VAL, int R, typename Up>
+__device__ __forceinline__ void sort_phase(uint32_t (&k)[R], uint32_t (&x)[R], int top, unsigned lane, Up up) {
+#pragma unroll
+    for (int stride = 16 * R; stride > 0; stride >>= 1) {
+        if (stride > top) continue;
+        if (stride >= R) {
+            const bool lower = (lane & (stride / R)) == 0;
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                const uint32_t pk = __shfl_xor_sync(KC_FULL_MASK, k[j], stride / R);
+                if (HAS_VAL) {
+                    const uint32_t px = __shfl_xor_sync(KC_FULL_MASK, x[j], stride / R);
+                    const bool take = lower ? pk < k[j] : pk > k[j];
+                    k[j] = take ? pk : k[j];
+                    x[j] = take ? px : x[j];
+                } else {
+                    k[j] = lower ? min(k[j], pk) : max(k[j], pk);
+                }
             }
+        } else {
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (!(j & stride)) sort_pair<HAS_VAL>(k[j], x[j], k[j | stride], x[j | stride], up(j));
         }
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) {
-            const uint32_t j = i / P, o = i % P;
-            const bool in = o < rlen[j];
-            sk[i] = in ? key[rstart[j] + o] : 0xffffffffu;
-            if (HAS_VAL) sv[i] = in ? val[rstart[j] + o] : 0xffffffffu;
+    }
+}
+
+template <bool HAS_VAL, int R, int W>
+__global__ void __launch_bounds__(SORT_THREADS) sort_rows_reg(const int64_t *__restrict__ rowptr,
+                                                              const uint32_t *__restrict__ rows, uint64_t nrows,
+                                                              uint32_t *key, uint32_t *val) {
+    constexpr int OWN = 32 * R;  // entries of a warp
+    constexpr int RPC = SORT_THREADS / 32 / W;  // rows per CTA
+    __shared__ uint32_t sk[SORT_THREADS / 32][OWN + R];
+    __shared__ uint32_t sv[HAS_VAL ? SORT_THREADS / 32 : 1][HAS_VAL ? OWN + R : 1];
+    const unsigned lane = threadIdx.x & 31, wib = threadIdx.x >> 5, w = wib % W;
+    for (uint64_t g = (uint64_t)blockIdx.x * RPC; g < nrows; g += (uint64_t)gridDim.x * RPC) {
+        const uint64_t r = g + wib / W;
+        int64_t start = 0;
+        uint32_t len = 0;
+        if (r < nrows) {
+            const uint32_t v = rows[r];
+            start = rowptr[v] + (int64_t)w * OWN;
+            const int64_t left = rowptr[v + 1] - start;
+            len = left <= 0 ? 0u : left < OWN ? (uint32_t)left : (uint32_t)OWN;
         }
-        __syncthreads();
-        for (uint32_t size = 2; size <= P; size <<= 1) {
-            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                for (uint32_t q = threadIdx.x; q < E / 2; q += blockDim.x) {
-                    const uint32_t i = 2 * stride * (q / stride) + (q % stride);
-                    const uint32_t j = i + stride;
-                    const bool asc = ((i & (P - 1)) & size) == 0;
-                    const uint32_t ki = sk[i], kj = sk[j];
-                    const uint32_t vi = HAS_VAL ? sv[i] : 0u, vj = HAS_VAL ? sv[j] : 0u;
-                    const bool sw = asc ? kv_less<HAS_VAL>(kj, vj, ki, vi) : kv_less<HAS_VAL>(ki, vi, kj, vj);
-                    if (sw) {
-                        sk[i] = kj;
-                        sk[j] = ki;
-                        if (HAS_VAL) {
-                            sv[i] = vj;
-                            sv[j] = vi;
-                        }
+        uint32_t k[R], x[R];
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const uint32_t e = j * 32 + lane;
+            k[j] = e < len ? key[start + e] : 0xffffffffu;
+            x[j] = HAS_VAL && e < len ? val[start + e] : 0xffffffffu;
+        }
+        // entries whose index has the bit `size` sort downwards in that phase
+#pragma unroll
+        for (int size = 2; size <= OWN; size <<= 1) {
+            uint32_t flip = 0;
+            if (size < OWN && size >= R) flip = (lane & (size / R)) ? 0xffffffffu : 0u;
+            if (size == OWN) flip = W > 1 && (w & 1) ? 0xffffffffu : 0u;
+#pragma unroll
+            for (int j = 0; j < R; j++) k[j] ^= flip;
+            sort_phase<HAS_VAL, R>(k, x, size / 2, lane, [&](int j) { return size >= R || !(j & size); });
+#pragma unroll
+            for (int j = 0; j < R; j++) k[j] ^= flip;
+        }
+        if constexpr (W > 1) {
+#pragma unroll 1
+            for (int ws = 2; ws <= W; ws <<= 1) {  // phases of 2, 4, .. W warps
+                const uint32_t flip = ws < W && (w & ws) ? 0xffffffffu : 0u;
+#pragma unroll
+                for (int j = 0; j < R; j++) k[j] ^= flip;
+#pragma unroll 1
+                for (int d = ws / 2; d > 0; d >>= 1) {
+                    const unsigned other = wib ^ d;
+                    const bool lower = (w & d) == 0;
+                    __syncthreads();
+#pragma unroll
+                    for (int j = 0; j < R; j++) {
+                        sk[wib][j * 32 + lane] = k[j];
+                        if (HAS_VAL) sv[wib][j * 32 + lane] = x[j];
+                    }
+                    __syncthreads();
+#pragma unroll
+                    for (int j = 0; j < R; j++) {
+                        const uint32_t pk = sk[other][j * 32 + lane];
+                        const bool take = lower ? pk < k[j] : pk > k[j];
+                        if (HAS_VAL) x[j] = take ? sv[other][j * 32 + lane] : x[j];
+                        k[j] = take ? pk : k[j];
                     }
                 }
-                __syncthreads();
+                sort_phase<HAS_VAL, R>(k, x, OWN / 2, lane, [](int) { return true; });
+#pragma unroll
+                for (int j = 0; j < R; j++) k[j] ^= flip;
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const uint32_t i = lane * R + j;
+            sk[wib][i + i / 32] = k[j];
+            if (HAS_VAL) sv[wib][i + i / 32] = x[j];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const uint32_t e = j * 32 + lane;
+            if (e < len) {
+                key[start + e] = sk[wib][e + j];
+                if (HAS_VAL) val[start + e] = sv[wib][e + j];
             }
         }
-        for (uint32_t i = threadIdx.x; i < E; i += blockDim.x) {
-            const uint32_t j = i / P, o = i % P;
-            if (o < rlen[j]) {
-                key[rstart[j] + o] = sk[i];
-                if (HAS_VAL) val[rstart[j] + o] = sv[i];
+        __syncwarp();
+    }
+}
+
+// Long rows that will be de-duplicated: the columns of a row set bits in a
+// shared-memory bitmap, which is then read back in order.  A row takes as
+// many passes as the columns need bitmaps; the slots freed by repeated
+// entries are filled with the row's last column, so the row stays sorted and
+// the de-duplication drops them.  Results of several passes wait in tk.  What
+// bounds it is clearing and reading the bitmap (about 4,500 clocks a pass);
+// the radix sort below takes about 7 clocks an entry of an SM, so rows of at
+// least BITMAP_ROW entries per pass go this way (R-MAT 22, rows above 4,096:
+// 2.42 ms by radix, 0.80 ms here).
+constexpr uint32_t BITMAP_WORDS = 49152;  // 192 KB: 1,572,864 columns a pass
+constexpr uint32_t BITMAP_ROW = 512;
+constexpr int BITMAP_THREADS = 1024;
+
+__global__ void __launch_bounds__(BITMAP_THREADS) sort_rows_bitmap(const int64_t *__restrict__ rowptr,
+                                                                   const uint32_t *__restrict__ rows, uint64_t nrows,
+                                                                   uint32_t n, uint32_t min_len, uint32_t *key,
+                                                                   uint32_t *tk) {
+    extern __shared__ __align__(16) uint32_t bits[];
+    __shared__ uint32_t wsum[BITMAP_THREADS / 32];
+    __shared__ uint32_t last_sh;
+    constexpr uint32_t STEP = 128;                                   // words a warp reads at once
+    constexpr uint32_t SEG = BITMAP_WORDS / (BITMAP_THREADS / 32);   // words of a warp
+    static_assert(SEG % STEP == 0, "a warp's words are whole steps");
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t cols = BITMAP_WORDS * 32;
+    for (uint64_t r = blockIdx.x; r < nrows; r += gridDim.x) {
+        const uint32_t v = rows[r];
+        const int64_t start = rowptr[v];
+        const uint32_t len = (uint32_t)(rowptr[v + 1] - start);
+        if (len < min_len) continue;
+        uint32_t *out = n > cols ? tk + start : key + start;
+        uint32_t off = 0;  // columns written
+        for (uint64_t c0 = 0; c0 < n; c0 += cols) {
+            for (uint32_t i = threadIdx.x; i < BITMAP_WORDS / 4; i += BITMAP_THREADS)
+                reinterpret_cast<uint4 *>(bits)[i] = make_uint4(0, 0, 0, 0);
+            __syncthreads();
+#pragma unroll 4
+            for (uint32_t j = threadIdx.x; j < len; j += BITMAP_THREADS) {
+                const uint64_t c = (uint64_t)key[start + j] - c0;  // wraps below c0
+                if (c < cols) atomicOr(&bits[c >> 5], 1u << (c & 31));
             }
+            __syncthreads();
+            uint32_t own = 0;
+            for (uint32_t i = warp * SEG + lane * 4; i < (warp + 1) * SEG; i += STEP) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(bits + i);
+                own += __popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w);
+            }
+            own = __reduce_add_sync(KC_FULL_MASK, own);
+            if (lane == 0) wsum[warp] = own;
+            __syncthreads();
+            const uint32_t mine = wsum[lane];  // 32 warps
+            uint32_t pos = off + __reduce_add_sync(KC_FULL_MASK, lane < warp ? mine : 0u);
+            off += __reduce_add_sync(KC_FULL_MASK, mine);
+            for (uint32_t i = warp * SEG + lane * 4; own && i < (warp + 1) * SEG; i += STEP) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(bits + i);
+                const uint32_t word[4] = {q.x, q.y, q.z, q.w};
+                uint32_t tot;
+                uint32_t at = pos + warp_excl_scan(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w), lane, tot);
+                pos += tot;
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    for (uint32_t b = word[t]; b; b &= b - 1) {
+                        const uint32_t c = (uint32_t)c0 + (i + t) * 32 + __ffs(b) - 1;
+                        out[at++] = c;
+                        if (at == off) last_sh = c;  // the last of this pass (the row's, after the last pass)
+                    }
+            }
+            __syncthreads();
         }
+        const uint32_t last = last_sh;
+        for (uint32_t j = off + threadIdx.x; j < len; j += BITMAP_THREADS) key[start + j] = last;
+        if (out != key + start)
+            for (uint32_t j = threadIdx.x; j < off; j += BITMAP_THREADS) key[start + j] = out[j];
         __syncthreads();
     }
 }
@@ -345,7 +505,7 @@ template <bool HAS_VAL>
 __global__ void __launch_bounds__(RADIX_THREADS) sort_rows_radix(const int64_t *__restrict__ rowptr,
                                                                  const uint32_t *__restrict__ rows, uint64_t nrows,
                                                                  uint32_t *key, uint32_t *val, uint32_t *tk,
-                                                                 uint32_t *tv, int passes) {
+                                                                 uint32_t *tv, int passes, uint32_t below) {
     __shared__ uint32_t hist[256];
     __shared__ uint32_t base[256];
     __shared__ uint32_t wcnt[RADIX_WARPS][256];
@@ -354,6 +514,7 @@ __global__ void __launch_bounds__(RADIX_THREADS) sort_rows_radix(const int64_t *
         uint32_t v = rows[r];
         int64_t start = rowptr[v];
         uint32_t len = (uint32_t)(rowptr[v + 1] - start);
+        if (len >= below) continue;  // sorted by sort_rows_bitmap
         uint32_t *ik = key + start, *iv = HAS_VAL ? val + start : nullptr;
         uint32_t *ok = tk + start, *ov = HAS_VAL ? tv + start : nullptr;
         for (int pass = 0; pass < passes; pass++) {
@@ -419,22 +580,37 @@ __global__ void __launch_bounds__(RADIX_THREADS) sort_rows_radix(const int64_t *
 }
 
 template <bool HAS_VAL>
-static void launch_pack(int logp, const int64_t *rowptr, const uint32_t *rows, uint64_t nrows, uint32_t *key,
-                        uint32_t *val, int sms, cudaStream_t s) {
-    const uint64_t rpc = logp >= 10 ? 1 : (SORT_PACK >> logp);
+static void launch_reg(int logp, const int64_t *rowptr, const uint32_t *rows, uint64_t nrows, uint32_t *key,
+                       uint32_t *val, int sms, cudaStream_t s) {
+    const uint64_t rpc = logp <= 10 ? SORT_THREADS / 32 : (SORT_THREADS / 32) >> (logp - 10);
     const int gr = (int)std::max<uint64_t>(1, std::min<uint64_t>((nrows + rpc - 1) / rpc, (uint64_t)sms * 8));
     switch (logp) {
-    case 6: sort_rows_pack<HAS_VAL, 6><<<gr, 256, 0, s>>>(rowptr, rows, nrows, key, val); break;
-    case 7: sort_rows_pack<HAS_VAL, 7><<<gr, 256, 0, s>>>(rowptr, rows, nrows, key, val); break;
-    case 8: sort_rows_pack<HAS_VAL, 8><<<gr, 256, 0, s>>>(rowptr, rows, nrows, key, val); break;
-    case 9: sort_rows_pack<HAS_VAL, 9><<<gr, 256, 0, s>>>(rowptr, rows, nrows, key, val); break;
-    case 10: sort_rows_pack<HAS_VAL, 10><<<gr, 256, 0, s>>>(rowptr, rows, nrows, key, val); break;
-    case 11: sort_rows_pack<HAS_VAL, 11><<<gr, 256, 0, s>>>(rowptr, rows, nrows, key, val); break;
-    default: sort_rows_pack<HAS_VAL, 12><<<gr, 256, 0, s>>>(rowptr, rows, nrows, key, val); break;
+    case 6: sort_rows_reg<HAS_VAL, 2, 1><<<gr, SORT_THREADS, 0, s>>>(rowptr, rows, nrows, key, val); break;
+    case 7: sort_rows_reg<HAS_VAL, 4, 1><<<gr, SORT_THREADS, 0, s>>>(rowptr, rows, nrows, key, val); break;
+    case 8: sort_rows_reg<HAS_VAL, 8, 1><<<gr, SORT_THREADS, 0, s>>>(rowptr, rows, nrows, key, val); break;
+    case 9: sort_rows_reg<HAS_VAL, 16, 1><<<gr, SORT_THREADS, 0, s>>>(rowptr, rows, nrows, key, val); break;
+    case 10: sort_rows_reg<HAS_VAL, HAS_VAL ? 16 : 32, HAS_VAL ? 2 : 1><<<gr, SORT_THREADS, 0, s>>>(rowptr, rows, nrows, key, val); break;
+    case 11: sort_rows_reg<HAS_VAL, HAS_VAL ? 16 : 32, HAS_VAL ? 4 : 2><<<gr, SORT_THREADS, 0, s>>>(rowptr, rows, nrows, key, val); break;
+    default: sort_rows_reg<HAS_VAL, HAS_VAL ? 16 : 32, HAS_VAL ? 8 : 4><<<gr, SORT_THREADS, 0, s>>>(rowptr, rows, nrows, key, val); break;
     }
 }
 
-static int sort_rows(Graph *g, uint32_t *key, uint32_t *val, uint32_t max_key, cudaStream_t s) {
+// Raises sort_rows_bitmap's dynamic shared-memory limit, once per device.
+static int bitmap_smem_limit() {
+    static std::mutex mu;
+    static bool done[64] = {};
+    int dev = 0;
+    KC_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(KC_ERR_INVALID, "device %d out of range", dev);
+    std::lock_guard<std::mutex> lk(mu);
+    if (done[dev]) return KC_OK;
+    KC_CUDA(cudaFuncSetAttribute(sort_rows_bitmap, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BITMAP_WORDS * 4)));
+    done[dev] = true;
+    return KC_OK;
+}
+
+// dedup: the rows' repeated entries will be dropped (keys only).
+static int sort_rows(Graph *g, uint32_t *key, uint32_t *val, uint32_t max_key, bool dedup, cudaStream_t s) {
     const uint32_t n = g->n;
     if (n == 0 || g->nnz == 0) return KC_OK;
     const int sms = current_sms();
@@ -461,8 +637,8 @@ static int sort_rows(Graph *g, uint32_t *key, uint32_t *val, uint32_t max_key, c
     }
     for (int c = 1; c < SORT_BUCKETS - 1; c++) {
         if (!h[c]) continue;
-        if (hv) launch_pack<true>(c + 5, g->rowptr, list + off[c], h[c], key, val, sms, s);
-        else launch_pack<false>(c + 5, g->rowptr, list + off[c], h[c], key, val, sms, s);
+        if (hv) launch_reg<true>(c + 5, g->rowptr, list + off[c], h[c], key, val, sms, s);
+        else launch_reg<false>(c + 5, g->rowptr, list + off[c], h[c], key, val, sms, s);
     }
     uint32_t *tk = nullptr, *tv = nullptr;
     int rc = KC_OK;
@@ -471,13 +647,21 @@ static int sort_rows(Graph *g, uint32_t *key, uint32_t *val, uint32_t max_key, c
         int bits = 1;
         while (bits < 32 && (max_key >> bits) != 0) bits++;
         int passes = (bits + 7) / 8;
-        rc = dalloc(&tk, g->nnz, "radix staging keys");
+        // rows from this length on go through the bitmap
+        const uint64_t maps = ((uint64_t)n + BITMAP_WORDS * 32 - 1) / (BITMAP_WORDS * 32);
+        const uint32_t bitmap_from = dedup && !hv ? (uint32_t)std::min<uint64_t>(maps * BITMAP_ROW, 0xffffffffu) : 0xffffffffu;
+        const bool all_bitmap = bitmap_from <= CLASS_B_MAX + 1;
+        if (!all_bitmap || maps > 1) rc = dalloc(&tk, g->nnz, "row sort staging keys");
         if (rc == KC_OK && hv) rc = dalloc(&tv, g->nnz, "radix staging values");
+        if (rc == KC_OK && bitmap_from != 0xffffffffu) rc = bitmap_smem_limit();
         if (rc == KC_OK) {
             const uint32_t *lc = list + off[SORT_BUCKETS - 1];
             int gr = (int)std::min<unsigned long long>(hc, (unsigned long long)sms * 4);
-            if (hv) sort_rows_radix<true><<<gr, RADIX_THREADS, 0, s>>>(g->rowptr, lc, hc, key, val, tk, tv, passes);
-            else sort_rows_radix<false><<<gr, RADIX_THREADS, 0, s>>>(g->rowptr, lc, hc, key, val, tk, tv, passes);
+            if (bitmap_from != 0xffffffffu)
+                sort_rows_bitmap<<<(unsigned)std::min<unsigned long long>(hc, (unsigned long long)sms), BITMAP_THREADS,
+                                   BITMAP_WORDS * 4, s>>>(g->rowptr, lc, hc, n, bitmap_from, key, tk);
+            if (hv) sort_rows_radix<true><<<gr, RADIX_THREADS, 0, s>>>(g->rowptr, lc, hc, key, val, tk, tv, passes, bitmap_from);
+            else if (!all_bitmap) sort_rows_radix<false><<<gr, RADIX_THREADS, 0, s>>>(g->rowptr, lc, hc, key, val, tk, tv, passes, bitmap_from);
         }
     }
     e = cudaGetLastError();
@@ -684,9 +868,9 @@ int build_csr_from_edges(Graph *g, const uint32_t *d_src, const uint32_t *d_dst,
     dfree(cur);
     if (e != cudaSuccess) { dfree(deg); dfree(err); dfree(key); return fail(KC_ERR_CUDA, "scatter: %s", cudaGetErrorString(e)); }
     if (keep_order) {
-        rc = sort_rows(g, key, g->col, (uint32_t)(2 * m), s);
+        rc = sort_rows(g, key, g->col, (uint32_t)(2 * m), false, s);
     } else {
-        rc = sort_rows(g, g->col, nullptr, n, s);
+        rc = sort_rows(g, g->col, nullptr, n, (flags & KC_EDGES_DEDUP) != 0, s);
     }
     dfree(key);
     if (rc) { dfree(deg); dfree(err); return rc; }
