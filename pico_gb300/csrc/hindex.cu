@@ -40,6 +40,14 @@
 //     support test is skipped and the histogram window is put under the
 //     bound, so sweep 0 gives rows up to 8,192 entries to warps.  On R-MAT
 //     graphs this reads about 40% fewer row entries;
+//   * what bounds a sweep is the dependent gathers of each vertex (its data, its
+//     row, the estimates, the notifications) and its end, where the last warps
+//     still hold vertices: a warp's vertices have their data read together,
+//     rows above 512 entries are handed out first and one by one in sweep 0 too,
+//     the shorter ones in smaller steps the fewer there are, and queued
+//     vertices leave a warp 32 at a time (Erdos-Renyi 10^6 / 8 x 10^6 1.94 ->
+//     1.20 ms, R-MAT 18 1.86 -> 1.35, R-MAT 22 7.45 -> 7.41, R-MAT 25 with a
+//     planted core 72.6 -> 67.2);
 //   * updates are visible at once within a sweep (Gauss-Seidel), which only
 //     shortens the trajectory; sweeps are separated by a grid barrier with a
 //     bounded wait.
@@ -54,7 +62,9 @@ constexpr int HX_THREADS = 512;
 constexpr int HX_WARPS = HX_THREADS / 32;
 constexpr uint32_t HX_WARP_MAX = 512;   // rows up to this length: one warp
 constexpr uint32_t HX_BINS = 4096;      // CTA histogram bins
-constexpr unsigned HX_GRAB = 8;         // short-row vertices a warp takes per cursor step
+constexpr int HX_STREAM = 4;  // row entries in flight per lane when a warp streams a long row (8: slower, spills)
+constexpr unsigned HX_GRAB = 8;   // short-row vertices a warp takes per cursor step, at most
+constexpr unsigned HX_TURNS = 2;  // steps each warp should get in a sweep, for an even end
 constexpr int HX_CACHE = 4;             // row entries per lane kept in registers (rows up to 32 * HX_CACHE)
 constexpr uint32_t HX_ORD_MIN = 32 * HX_CACHE;  // the shortest rows that can get an ordered copy are longer
 constexpr uint32_t HX_ORD_WARP = 8192;  // the copy of a row up to this length is made by one warp
@@ -86,25 +96,27 @@ struct HxArgs {
 __device__ __forceinline__ unsigned hx_bucket(uint32_t x) { return x ? 31u - __clz(x) : 0u; }
 
 // Estimates start at the degrees; rows above sweep0_rows entries are queued
-// for the CTAs of sweep 0.  With ord_rows, the rows above ord_min entries
+// for the CTAs of sweep 0, the other rows above HX_WARP_MAX (at the far end of
+// list0) for single warps, before the rest.  With ord_rows, the rows above ord_min entries
 // are listed for the ordered copy: up to HX_ORD_WARP entries from the front
 // of ord_rows (long-row index p), longer ones from its far end (index
 // max_long - 1 - q), each with its index in lid, and vb holds every
 // vertex's degree bucket (one byte: the copies gather these, not degrees).
 __global__ void hindex_init(const int64_t *__restrict__ rowptr, uint32_t n, uint32_t *c, uint32_t *inlist0,
-                            uint32_t *inlist1, uint32_t *big0, uint32_t sweep0_rows, uint32_t *ord_rows,
+                            uint32_t *inlist1, uint32_t *list0, uint32_t *big0, uint32_t sweep0_rows, uint32_t *ord_rows,
                             uint32_t *lid, uint8_t *vb, uint32_t ord_min, uint64_t max_long, HindexCtl *ctl) {
     const unsigned lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < n; base += stride) {
         uint64_t v = base + threadIdx.x;
-        bool bigv = false, midl = false, hugel = false;
+        bool bigv = false, medv = false, midl = false, hugel = false;
         if (v < n) {
             uint32_t d = (uint32_t)(rowptr[v + 1] - rowptr[v]);
             c[v] = d;
             if (vb) vb[v] = (uint8_t)hx_bucket(d);
             bigv = d > sweep0_rows;
+            medv = d > HX_WARP_MAX && !bigv;
             midl = ord_rows && d > ord_min && d <= HX_ORD_WARP;
             hugel = ord_rows && d > ord_min && d > HX_ORD_WARP;
         }
@@ -114,6 +126,13 @@ __global__ void hindex_init(const int64_t *__restrict__ rowptr, uint32_t n, uint
             if (lane == 0) p = atomicAdd(&ctl->big_len[0], (unsigned long long)__popc(b));
             p = __shfl_sync(KC_FULL_MASK, p, 0);
             if (bigv) big0[p + __popc(b & lt)] = (uint32_t)v;
+        }
+        const unsigned bd = __ballot_sync(KC_FULL_MASK, medv);
+        if (bd) {
+            unsigned long long p = 0;
+            if (lane == 0) p = atomicAdd(&ctl->mid_len[0], (unsigned long long)__popc(bd));
+            p = __shfl_sync(KC_FULL_MASK, p, 0);
+            if (medv) list0[n - (p + __popc(bd & lt))] = (uint32_t)v;
         }
         const unsigned bm = __ballot_sync(KC_FULL_MASK, midl);
         if (bm) {
@@ -264,41 +283,59 @@ __global__ void __launch_bounds__(HX_ORD_THREADS) hx_order_rows(const int64_t *_
     }
 }
 
-// Queue u for the next sweep (list and bitmap of parity nxt) unless it is
-// queued already.  Vertices pending in the current sweep are queued again: a
-// notification never relies on an evaluation still to come in this sweep,
-// which could read the neighbour's estimate before its update is visible.
-// Rows up to A.warp_rows entries (tunable "hindex.warp_rows") go to the warp list: one warp streams
-// such a row with fewer synchronisations than a CTA.  Rows above
-// HX_WARP_MAX entries are kept apart and handed out first, one per warp, so
-// that the short rows even out the end of the sweep.
-__device__ __forceinline__ void hx_activate(const HxArgs &A, uint32_t u, unsigned nxt) {
-    unsigned bit = 1u << (u & 31);
-    if (__ldcg(&A.inlist[nxt][u >> 5]) & bit) return;
-    unsigned old = atomicOr(&A.inlist[nxt][u >> 5], bit);
-    if (old & bit) return;
-    uint32_t d = (uint32_t)(A.rowptr[u + 1] - A.rowptr[u]);
-    if (d > A.warp_rows) {
-        unsigned long long p = atomicAdd(&A.ctl->big_len[nxt], 1ull);
-        A.big[nxt][p] = u;
-    } else if (d > HX_WARP_MAX) {
-        // medium rows fill the list from its far end (a vertex is listed
-        // once, so both ends together hold at most n entries)
-        unsigned long long p = atomicAdd(&A.ctl->mid_len[nxt], 1ull);
-        A.list[nxt][A.n - p] = u;
-    } else {
-        unsigned long long p = atomicAdd(&A.ctl->list_len[nxt], 1ull);
-        A.list[nxt][p] = u;
+// A warp's vertices for the next sweep's list of short rows, kept in shared
+// memory until there are 32 of them: one atomicAdd on the list's length and one
+// coalesced store per 32 vertices.  (Every lowered vertex queues itself, and one
+// atomicAdd per vertex on that one counter held the early sweeps back.)
+struct HxStage {
+    uint32_t *buf;  // 64 entries
+    unsigned cnt;   // the same on every lane, below 32 between calls
+};
+
+__device__ __forceinline__ void hx_stage_push(const HxArgs &A, HxStage &st, bool take, uint32_t u, unsigned nxt,
+                                              unsigned lane) {
+    const unsigned m = __ballot_sync(KC_FULL_MASK, take);
+    if (!m) return;
+    if (take) st.buf[st.cnt + __popc(m & ((1u << lane) - 1u))] = u;
+    st.cnt += __popc(m);
+    if (st.cnt >= 32) {
+        __syncwarp();
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(&A.ctl->list_len[nxt], 32ull);
+        base = __shfl_sync(KC_FULL_MASK, base, 0);
+        A.list[nxt][base + lane] = st.buf[lane];
+        const uint32_t left = st.buf[32 + lane];
+        __syncwarp();
+        st.buf[lane] = left;
+        st.cnt -= 32;
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ void hx_stage_flush(const HxArgs &A, HxStage &st, unsigned nxt, unsigned lane) {
+    if (st.cnt) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(&A.ctl->list_len[nxt], (unsigned long long)st.cnt);
+        base = __shfl_sync(KC_FULL_MASK, base, 0);
+        if (lane < st.cnt) A.list[nxt][base + lane] = st.buf[lane];
+        st.cnt = 0;
+        __syncwarp();
     }
 }
 
-// hx_activate for K candidates per lane (u[k] where cand[k]), warp-wide:
-// every lane calls it.  The pending-bit reads, the claiming atomicOr, the
-// row-length reads and the list appends of all K candidates are each in
-// flight together, and the appends to each list take one atomicAdd per warp.
+// Queue K candidates per lane (u[k] where cand[k]) for the next sweep (list and
+// bitmap of parity nxt) unless they are queued already; warp-wide: every lane
+// calls it.  Vertices pending in the current sweep are queued again: a
+// notification never relies on an evaluation still to come in this sweep,
+// which could read the neighbour's estimate before its update is visible.
+// Rows up to A.warp_rows entries (tunable "hindex.warp_rows") go to the warp
+// list: one warp streams such a row with fewer synchronisations than a CTA.
+// Rows above HX_WARP_MAX entries are kept apart and handed out first, one per
+// warp, so that the short rows even out the end of the sweep.  The pending-bit
+// reads of all K candidates travel together, then the claiming atomicOr.
 template <int K>
 __device__ __forceinline__ void hx_activate_all(const HxArgs &A, const uint32_t (&u)[K], const bool (&cand)[K],
-                                                unsigned nxt, unsigned lane) {
+                                                unsigned nxt, unsigned lane, HxStage &st) {
     bool anyc = false;
 #pragma unroll
     for (int k = 0; k < K; k++) anyc |= cand[k];
@@ -310,33 +347,28 @@ __device__ __forceinline__ void hx_activate_all(const HxArgs &A, const uint32_t 
     unsigned old[K];
 #pragma unroll
     for (int k = 0; k < K; k++) old[k] = need[k] ? atomicOr(&A.inlist[nxt][u[k] >> 5], 1u << (u[k] & 31)) : ~0u;
-    int kind[K];  // -1: nothing to queue; 0 short, 1 medium, 2 long row
 #pragma unroll
     for (int k = 0; k < K; k++) {
-        kind[k] = -1;
-        if (!(old[k] & (1u << (u[k] & 31)))) {
+        const bool take = need[k] && !(old[k] & (1u << (u[k] & 31)));
+        int kind = take ? 0 : -1;  // -1: nothing to queue; 0 short, 1 medium, 2 long row
+        if (take) {
             const int64_t d = A.rowptr[u[k] + 1] - A.rowptr[u[k]];
-            kind[k] = d > (int64_t)A.warp_rows ? 2 : d > (int64_t)HX_WARP_MAX ? 1 : 0;
+            kind = d > (int64_t)A.warp_rows ? 2 : d > (int64_t)HX_WARP_MAX ? 1 : 0;
         }
-    }
-    const unsigned lt = (1u << lane) - 1u;
+        hx_stage_push(A, st, kind == 0, u[k], nxt, lane);
+        if (!__any_sync(KC_FULL_MASK, kind > 0)) continue;
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-        if (!__any_sync(KC_FULL_MASK, kind[k] >= 0)) continue;
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const unsigned m = __ballot_sync(KC_FULL_MASK, kind[k] == q);
+        for (int q = 1; q < 3; q++) {
+            const unsigned m = __ballot_sync(KC_FULL_MASK, kind == q);
             if (!m) continue;
             unsigned long long base = 0;
             if (lane == __ffs(m) - 1)
-                base = atomicAdd(q == 2 ? &A.ctl->big_len[nxt] : q == 1 ? &A.ctl->mid_len[nxt] : &A.ctl->list_len[nxt],
-                                 (unsigned long long)__popc(m));
+                base = atomicAdd(q == 2 ? &A.ctl->big_len[nxt] : &A.ctl->mid_len[nxt], (unsigned long long)__popc(m));
             base = __shfl_sync(KC_FULL_MASK, base, __ffs(m) - 1);
-            if (kind[k] == q) {
-                const unsigned long long p = base + __popc(m & lt);
+            if (kind == q) {
+                const unsigned long long p = base + __popc(m & ((1u << lane) - 1u));
                 if (q == 2) A.big[nxt][p] = u[k];
-                else if (q == 1) A.list[nxt][A.n - p] = u[k];
-                else A.list[nxt][p] = u[k];
+                else A.list[nxt][A.n - p] = u[k];  // from the far end (a vertex is listed once, so both ends fit)
             }
         }
     }
@@ -424,8 +456,6 @@ __device__ __forceinline__ uint32_t hx_warp_lower(const HxRow &R, const uint32_t
     }
 }
 
-constexpr int HX_STREAM = 4;  // row entries in flight per lane when a warp streams a long row (8: slower, spills)
-
 // Add the estimates of row entries [j0, j1) to the window [lo, cap) of
 // hist (bin x - lo) and count those at or above cap, starting from cnt.
 // Stops early once the count reaches stop (stop = 0: the whole range).
@@ -453,20 +483,39 @@ __device__ __forceinline__ uint32_t hx_warp_gather(const uint32_t *row, const ui
     return cnt;
 }
 
-// One warp: recompute vertex v (any row length; long rows are streamed).
+// A vertex to examine, with what every examination reads first: its row, its
+// estimate (only its own examination lowers it, so it may be read ahead) and,
+// where the row has an ordered copy, its long-row index.
+struct HxVertex {
+    uint32_t v, cap, lid, len;
+    int64_t s;
+};
+
+// Reads a vertex's data and clears its pending bit (clear): this sweep's bitmap
+// is cleared as its vertices are taken, so it is empty when it becomes the next
+// sweep's.
+__device__ __forceinline__ HxVertex hx_load(const HxArgs &A, uint32_t v, unsigned cur, bool clear) {
+    HxVertex x;
+    x.v = v;
+    x.s = A.rowptr[v];
+    x.len = (uint32_t)(A.rowptr[v + 1] - x.s);
+    x.cap = __ldcg(&A.c[v]);
+    x.lid = A.ord && x.len > A.ord_min ? A.lid[v] : 0u;
+    if (clear) atomicAnd(&A.inlist[cur][v >> 5], ~(1u << (v & 31)));
+    return x;
+}
+
+// One warp: recompute vertex x.v (any row length; long rows are streamed).
 // hist: this warp's HX_WARP_MAX+1 shared bins.  Returns true if c[v] dropped.
 // Rows of at most HX_CACHE * 32 entries keep their neighbour ids and
 // estimates in registers: one gather pass serves the support test, the
 // histogram and the neighbour notification.  Longer rows run the support
 // test in chunks of HX_CACHE * 32 entries and stop once it holds.
-__device__ bool hx_warp_vertex(const HxArgs &A, uint32_t v, unsigned cur, bool clear, uint32_t *hist,
-                               unsigned lane) {
+__device__ bool hx_warp_vertex(const HxArgs &A, const HxVertex &x, unsigned cur, uint32_t *hist, unsigned lane,
+                               HxStage &st) {
     const unsigned nxt = cur ^ 1u;
-    const int64_t s = A.rowptr[v], e = A.rowptr[v + 1];
-    // this sweep's bitmap is cleared as its vertices are examined, so it is
-    // empty when it becomes the next sweep's
-    if (clear && lane == 0) atomicAnd(&A.inlist[cur][v >> 5], ~(1u << (v & 31)));
-    const uint32_t cap = __ldcg(&A.c[v]);
+    const uint32_t v = x.v, cap = x.cap;
+    const int64_t s = x.s, e = x.s + x.len;
     if (cap == 0) return false;
     const bool cached = e - s <= 32 * HX_CACHE;
     HxRow R;
@@ -474,7 +523,7 @@ __device__ bool hx_warp_vertex(const HxArgs &A, uint32_t v, unsigned cur, bool c
     R.e = e;
     R.ordered = A.ord != nullptr && e - s > (int64_t)A.ord_min;  // never a cached row
     R.r = R.ordered ? A.ord : A.col;
-    R.pf = R.ordered ? A.pref[(size_t)A.lid[v] * 32 + lane] : 0u;
+    R.pf = R.ordered ? A.pref[(size_t)x.lid * 32 + lane] : 0u;
     uint32_t cu[HX_CACHE], cv[HX_CACHE];
     uint32_t cnt = 0;
     uint32_t lo = 0;      // lowest value the histogram window covers
@@ -554,14 +603,26 @@ __device__ bool hx_warp_vertex(const HxArgs &A, uint32_t v, unsigned cur, bool c
     // An estimate read earlier in this call is at least the current one; it
     // can differ only if u was lowered concurrently in this sweep, and such a
     // u re-examines itself in the next sweep (below), after this write.
+    // A neighbour lowered in this sweep may have read c[v] before this write
+    // and skipped v (its window test saw the old, higher value) while this
+    // call counted it at its old estimate: v re-examines itself next sweep
+    // (lane 0's last candidate).
     if (cached) {
         bool cand[HX_CACHE];
 #pragma unroll
         for (int k = 0; k < HX_CACHE; k++) cand[k] = cu[k] != 0xffffffffu && cv[k] > h && cv[k] <= cap;
-        hx_activate_all(A, cu, cand, nxt, lane);
+        hx_activate_all(A, cu, cand, nxt, lane, st);
+        const uint32_t us[1] = {v};
+        const bool cs[1] = {lane == 0};
+        hx_activate_all(A, us, cs, nxt, lane, st);
     } else {
         // candidates have degree > h: an ordered row is read that far
         const int64_t en = R.end(h + 1);
+        {
+            const uint32_t uu[1] = {v};
+            const bool cand[1] = {lane == 0};
+            hx_activate_all(A, uu, cand, nxt, lane, st);
+        }
         for (int64_t jw = s; jw < en; jw += 32 * HX_STREAM) {  // warp-uniform trip count
             uint32_t uu[HX_STREAM], xx[HX_STREAM];
 #pragma unroll
@@ -574,13 +635,9 @@ __device__ bool hx_warp_vertex(const HxArgs &A, uint32_t v, unsigned cur, bool c
             bool cand[HX_STREAM];
 #pragma unroll
             for (int k = 0; k < HX_STREAM; k++) cand[k] = uu[k] != 0xffffffffu && xx[k] > h && xx[k] <= cap;
-            hx_activate_all(A, uu, cand, nxt, lane);
+            hx_activate_all(A, uu, cand, nxt, lane, st);
         }
     }
-    // A neighbour lowered in this sweep may have read c[v] before this write
-    // and skipped v (its window test saw the old, higher value) while this
-    // call counted it at its old estimate: v re-examines itself next sweep.
-    if (lane == 0) hx_activate(A, v, nxt);
     return true;
 }
 
@@ -592,18 +649,12 @@ __device__ bool hx_warp_vertex(const HxArgs &A, uint32_t v, unsigned cur, bool c
 // Returns the number of estimates lowered (the same on every lane).
 constexpr uint32_t HX_TINY = 32;
 
-__device__ unsigned hx_warp_tiny(const HxArgs &A, uint32_t vg, bool valid, unsigned cur, bool clear,
-                                 uint32_t *hist, unsigned lane) {
+__device__ unsigned hx_warp_tiny(const HxArgs &A, const HxVertex &x, bool valid, unsigned cur, uint32_t *hist,
+                                 unsigned lane, HxStage &st) {
     const unsigned nxt = cur ^ 1u;
     const unsigned gi = lane >> 3, gl = lane & 7;
-    int64_t s = 0, e = 0;
-    uint32_t cap = 0;
-    if (valid) {
-        s = A.rowptr[vg];
-        e = A.rowptr[vg + 1];
-        if (clear && gl == 0) atomicAnd(&A.inlist[cur][vg >> 5], ~(1u << (vg & 31)));
-        cap = __ldcg(&A.c[vg]);
-    }
+    const uint32_t vg = x.v, cap = valid ? x.cap : 0u;
+    const int64_t s = x.s, e = valid ? x.s + x.len : x.s;
     uint32_t cu[4], cv[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -665,8 +716,10 @@ __device__ unsigned hx_warp_tiny(const HxArgs &A, uint32_t vg, bool valid, unsig
     bool cand[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) cand[k] = low && cu[k] != 0xffffffffu && cv[k] > h && cv[k] <= cap;
-    hx_activate_all(A, cu, cand, nxt, lane);
-    if (low && gl == 0) hx_activate(A, vg, nxt);
+    hx_activate_all(A, cu, cand, nxt, lane, st);
+    const uint32_t us[1] = {vg};
+    const bool cs[1] = {low && gl == 0};
+    hx_activate_all(A, us, cs, nxt, lane, st);
     return (unsigned)__popc(__ballot_sync(KC_FULL_MASK, low && gl == 0));
 }
 
@@ -736,7 +789,8 @@ __device__ int hx_block_suffix_find(const uint32_t *hist, int nb, uint64_t base,
 }
 
 // One CTA: recompute vertex v with a long row.
-__device__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint32_t *hist, uint32_t *red) {
+__device__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint32_t *hist, uint32_t *red,
+                                HxStage &st) {
     const int64_t s = A.rowptr[v], e = A.rowptr[v + 1];
     __shared__ uint32_t cap_sh;
     __shared__ uint32_t pref_sh[32];  // ordered row: entries in degree buckets >= b
@@ -882,10 +936,14 @@ __device__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint3
             bool cand[HX_CACHE];
 #pragma unroll
             for (int k = 0; k < HX_CACHE; k++) cand[k] = uu[k] != 0xffffffffu && xx[k] > h && xx[k] <= cap;
-            hx_activate_all(A, uu, cand, nxt, lane);
+            hx_activate_all(A, uu, cand, nxt, lane, st);
+        }
+        if (warp == 0) {
+            const uint32_t uu[1] = {v};
+            const bool cand[1] = {lane == 0};
+            hx_activate_all(A, uu, cand, nxt, lane, st);
         }
     }
-    if (threadIdx.x == 0) hx_activate(A, v, nxt);
     __syncthreads();
     return true;
 }
@@ -896,11 +954,14 @@ constexpr uint32_t HX_SMEM_WORDS =
 __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
     __shared__ uint32_t hist[HX_SMEM_WORDS];
     __shared__ uint32_t red[HX_WARPS];
+    __shared__ uint32_t stage_sh[HX_WARPS][64];
+    __shared__ HxVertex grab_sh[HX_WARPS][HX_GRAB];  // the data of the vertices a warp has taken
     __shared__ unsigned int changed_sh;  // estimates this CTA lowered in the sweep
     __shared__ unsigned long long item_sh;
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     HindexCtl *ctl = A.ctl;
     const unsigned G = gridDim.x;
+    HxStage st = {stage_sh[warp], 0u};
     if (A.withhold && blockIdx.x == 0) {
         // The barrier count never reaches the grid size: the other CTAs' waits
         // run into their limit.  This CTA waits (bounded) for their verdict.
@@ -924,12 +985,12 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
         const unsigned long long t_sweep = tr ? global_ns() : 0ull;
         const bool all = sweep == 0 && A.first_all;
         const unsigned long long nsmall = all ? (unsigned long long)A.n : ld_relaxed64(&ctl->list_len[cur]);
-        const unsigned long long nmid = all ? 0ull : ld_relaxed64(&ctl->mid_len[cur]);
+        const unsigned long long nmid = ld_relaxed64(&ctl->mid_len[cur]);
         const unsigned long long nbig = ld_relaxed64(&ctl->big_len[cur]);
         if (tr && blockIdx.x == 0 && threadIdx.x == 0) {
             A.trace[sweep].t_start_ns = t_sweep;
             A.trace[sweep].level = sweep;
-            A.trace[sweep].scan_len = (unsigned)(nsmall + nmid);
+            A.trace[sweep].scan_len = (unsigned)(all ? nsmall : nsmall + nmid);  // sweep 0: all of them
             A.trace[sweep].spilled = (unsigned)nbig;
         }
         // long rows: one CTA each, taken dynamically
@@ -942,7 +1003,7 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
             uint32_t v = A.big[cur][i];
             if (!all && threadIdx.x == 0) atomicAnd(&A.inlist[cur][v >> 5], ~(1u << (v & 31)));
             __syncthreads();
-            const bool low = hx_block_vertex(A, v, nxt, hist, red);
+            const bool low = hx_block_vertex(A, v, nxt, hist, red, st);
             if (low && threadIdx.x == 0) changed_sh++;
             if (tr && threadIdx.x == 0) {
                 const int64_t len = A.rowptr[v + 1] - A.rowptr[v];
@@ -955,6 +1016,8 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
         // medium rows, one per warp, then short rows, HX_GRAB consecutive
         // entries at a time, each taken from a shared cursor; sweep 0 covers
         // every short row
+        const unsigned long long share = nsmall / ((unsigned long long)G * HX_WARPS * HX_TURNS);
+        const unsigned grab = share >= HX_GRAB ? HX_GRAB : share >= 3 ? 4u : share > 0 ? (unsigned)share : 1u;
         uint32_t *wh = hist + warp * (HX_WARP_MAX + 1);
         unsigned wchanged = 0;
         while (nmid) {
@@ -962,26 +1025,29 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
             if (lane == 0) i = atomicAdd(&ctl->mid_cursor, 1ull);
             i = __shfl_sync(KC_FULL_MASK, i, 0);
             if (i >= nmid) break;
-            wchanged += hx_warp_vertex(A, A.list[cur][A.n - i], cur, true, wh, lane) ? 1u : 0u;
+            const HxVertex x = hx_load(A, A.list[cur][A.n - i], cur, !all && lane == 0);
+            wchanged += hx_warp_vertex(A, x, cur, wh, lane, st) ? 1u : 0u;
         }
         for (;;) {
             unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(&ctl->cursor, (unsigned long long)HX_GRAB);
+            if (lane == 0) base = atomicAdd(&ctl->cursor, (unsigned long long)grab);
             base = __shfl_sync(KC_FULL_MASK, base, 0);
             if (base >= nsmall) break;
-            const unsigned cntv = (unsigned)(nsmall - base < HX_GRAB ? nsmall - base : HX_GRAB);
-            // the grab's vertices and row lengths on lanes 0..cntv-1; rows
-            // of at most HX_TINY entries go four at a time, the others one
-            // per warp (sweep 0 leaves rows above A.sweep0_rows to the CTAs)
-            uint32_t vi = 0;
-            int64_t di = 0;
+            const unsigned cntv = (unsigned)(nsmall - base < grab ? nsmall - base : grab);
+            // the grab's vertices and their data on lanes 0..cntv-1, read
+            // together; rows of at most HX_TINY entries go four at a time, the
+            // others one per warp (in sweep 0, rows above HX_WARP_MAX were
+            // taken above)
+            uint32_t len = 0;
             if (lane < cntv) {
-                vi = all ? (uint32_t)(base + lane) : A.list[cur][base + lane];
-                di = A.rowptr[vi + 1] - A.rowptr[vi];
+                const HxVertex x = hx_load(A, all ? (uint32_t)(base + lane) : A.list[cur][base + lane], cur, !all);
+                grab_sh[warp][lane] = x;
+                len = x.len;
             }
-            const bool in = lane < cntv && !(all && di > (int64_t)A.sweep0_rows);
-            unsigned tinym = __ballot_sync(KC_FULL_MASK, in && di <= (int64_t)HX_TINY);
-            unsigned restm = __ballot_sync(KC_FULL_MASK, in && di > (int64_t)HX_TINY);
+            __syncwarp();
+            const bool in = lane < cntv && !(all && len > HX_WARP_MAX);
+            unsigned tinym = __ballot_sync(KC_FULL_MASK, in && len <= HX_TINY);
+            unsigned restm = __ballot_sync(KC_FULL_MASK, in && len > HX_TINY);
             while (tinym) {
                 int pick = -1;  // this lane's group takes the (lane / 8)-th remaining tiny vertex
 #pragma unroll
@@ -990,16 +1056,16 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
                     if (g2 == (lane >> 3)) pick = p;
                     tinym &= tinym - 1u;
                 }
-                const uint32_t vg = __shfl_sync(KC_FULL_MASK, vi, pick < 0 ? 0 : pick);
-                wchanged += hx_warp_tiny(A, vg, pick >= 0, cur, !all, wh, lane);
+                wchanged += hx_warp_tiny(A, grab_sh[warp][pick < 0 ? 0 : pick], pick >= 0, cur, wh, lane, st);
             }
             while (restm) {
                 const int p = __ffs(restm) - 1;
                 restm &= restm - 1u;
-                const uint32_t v = __shfl_sync(KC_FULL_MASK, vi, p);
-                wchanged += hx_warp_vertex(A, v, cur, !all, wh, lane) ? 1u : 0u;
+                wchanged += hx_warp_vertex(A, grab_sh[warp][p], cur, wh, lane, st) ? 1u : 0u;
             }
+            __syncwarp();
         }
+        hx_stage_flush(A, st, nxt, lane);
         if (lane == 0 && wchanged) atomicAdd(&changed_sh, wchanged);
         __syncthreads();
         if (threadIdx.x == 0 && changed_sh) atomicOr(&ctl->changed, 1u);
@@ -1200,7 +1266,7 @@ int hindex_run(Graph *g, cudaStream_t s, kc_stats *st) {
     const int ig = std::max(1, std::min<int>(g->sm_count * 8, (int)((g->n + 255) / 256)));
     // the ordered copies of the long rows (part of every decomposition's
     // time); list[1] holds the rows to copy until sweep 0 queues vertices there
-    hindex_init<<<ig, 256, 0, s>>>(g->rowptr, g->n, g->core, g->bitmap, g->hx_bitmap, g->big[0],
+    hindex_init<<<ig, 256, 0, s>>>(g->rowptr, g->n, g->core, g->bitmap, g->hx_bitmap, g->list[0], g->big[0],
                                    sweep0_rows(g, ordered), ordered ? g->list[1] : nullptr, g->hx_lid,
                                    ordered ? g->hx_vb : nullptr, order_min(g), max_long_rows(g), g->hctl);
     if (ordered)
