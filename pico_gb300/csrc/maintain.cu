@@ -2,10 +2,10 @@
 //
 // The reference has no edge-update path (its "dyn" drivers only use dynamic
 // work queues); this subsystem is new.  Core numbers stay exact:
-//   * the CSR is rewritten in one streaming pass per change set: every row
-//     keeps its entries minus the deleted ones plus the inserted ones, sorted
-//     (binary searches in the small per-row change lists give every entry's
-//     output position directly);
+//   * the CSR is rewritten in one streaming pass per change set: the sorted
+//     change lists become edits of the column array (entries that go, entries
+//     that come before a position), and binary searches among the few edits
+//     near an entry give its new place;
 //   * deletions: cores only decrease, so the old cores are upper bounds; the
 //     h-index iteration restarts from them with the endpoints of the deleted
 //     edges active and converges to the new cores (only vertices whose
@@ -37,211 +37,360 @@ static int grid_of(const Graph *g, uint64_t items) {
     return (int)std::max<uint64_t>(1, std::min(b, cap));
 }
 
-__device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *a, uint32_t len, uint32_t x) {
-    uint32_t lo = 0, hi = len;
+// Entries of the ascending a[0..len) below x.
+template <class T>
+__device__ __forceinline__ uint64_t count_below(const T *__restrict__ a, uint64_t len, T x) {
+    uint64_t lo = 0, hi = len;
     while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (a[mid] < x) lo = mid + 1;
+        const uint64_t mid = (lo + hi) >> 1;
+        if (__ldg(&a[mid]) < x) lo = mid + 1;
         else hi = mid;
     }
     return lo;
 }
 
-// Every row: new length = old length, no changes yet; flags the rows that
-// the change lists touch.
-__global__ void mark_changed(const int64_t *__restrict__ rowptr, uint32_t n, const int64_t *__restrict__ drp,
-                             const int64_t *__restrict__ irp, uint32_t *dcnt, uint32_t *icnt, uint32_t *newlen,
-                             uint32_t *flag) {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
-        newlen[v] = (uint32_t)(rowptr[v + 1] - rowptr[v]);
-        if (dcnt) dcnt[v] = 0;
-        if (icnt) icnt[v] = 0;
-        const bool ch = (drp && drp[v + 1] != drp[v]) || (irp && irp[v + 1] != irp[v]);
-        flag[v] = ch ? 1u : 0u;
-    }
-}
-
-__global__ void list_changed(const uint32_t *__restrict__ flag, const int64_t *__restrict__ pos, uint32_t n,
-                             uint32_t *changed) {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
-        if (flag[v]) changed[pos[v]] = (uint32_t)v;
-}
-
-// Plans the changed rows (one warp per listed row): positions of deleted
-// entries, inserted values not already present, new row lengths.
-__global__ void merge_plan(const int64_t *__restrict__ rowptr, const uint32_t *__restrict__ col,
-                           const uint32_t *__restrict__ changed, uint32_t nchanged,
-                           const int64_t *__restrict__ drp, const uint32_t *__restrict__ dcol,
-                           const int64_t *__restrict__ irp, const uint32_t *__restrict__ icol, uint32_t *dpos,
-                           uint32_t *dcnt, uint32_t *ival, uint32_t *icnt, uint32_t *newlen,
-                           unsigned long long *applied) {
+// The same by a warp, 32 probes at a time: three dependent reads for lists of
+// up to 32,768 edits instead of fifteen, which is what a CTA of the rewrite
+// waits for before it can start.
+template <class T>
+__device__ __forceinline__ uint64_t warp_count_below(const T *__restrict__ a, uint64_t len, T x) {
     const unsigned lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    unsigned long long nd = 0, ni = 0;
-    for (uint64_t ci = warp; ci < nchanged; ci += nw) {
-        const uint32_t v = changed[ci];
-        const int64_t r0 = rowptr[v];
-        const uint32_t len = (uint32_t)(rowptr[v + 1] - r0);
-        const int64_t d0 = drp ? drp[v] : 0, i0 = irp ? irp[v] : 0;
-        const uint32_t dl = drp ? (uint32_t)(drp[v + 1] - d0) : 0u;
-        const uint32_t il = irp ? (uint32_t)(irp[v + 1] - i0) : 0u;
-        if (dl == 0 && il == 0) {
-            if (lane == 0) {
-                newlen[v] = len;
-                if (dcnt) dcnt[v] = 0;
-                if (icnt) icnt[v] = 0;
+    uint64_t lo = 0, hi = len;
+    while (hi - lo > 32) {
+        const uint64_t step = (hi - lo + 31) / 32, p = lo + lane * step + step - 1;  // the last entry of part `lane`
+        lo += step * __popc(__ballot_sync(KC_FULL_MASK, p < hi && __ldg(&a[p]) < x));
+        if (lo > hi) lo = hi;
+        if (hi - lo > step) hi = lo + step;
+    }
+    const uint64_t p = lo + lane;
+    return lo + __popc(__ballot_sync(KC_FULL_MASK, p < hi && __ldg(&a[p]) < x));
+}
+
+// ------------------------------------------------------------ change lists ----
+// A change list is its directed entries (row << 32 | column, both directions of
+// every listed edge) in ascending order; self-loops and padding are ~0 and come
+// last.  Index 0 below is the deletions, 1 the insertions.
+constexpr int CH_TILE = 2048;  // entries sorted by one CTA
+// Up to this many entries a list is sorted by tiles that rank their entries in
+// each other; longer ones go through the CSR builder, whose passes over all
+// vertices and dozens of launches then weigh less than the ranking, which
+// grows with the square.  Two updates of R-MAT 18 / 20 / 22, tiles against
+// builder: 130,000 entries 4.17 / 7.48 / 9.67 against 4.52 / 7.80 / 10.30 ms,
+// 260,000 entries the same within 2%, 520,000 entries (18, 22) 6.60 / 15.4
+// against 4.89 / 13.9 ms.
+constexpr uint64_t CH_TILED_MAX = 1ull << 17;
+
+struct ChangeLists {
+    const uint32_t *src[2], *dst[2];
+    uint64_t m[2];           // listed edges
+    unsigned tiles[2];       // of CH_TILE entries
+    unsigned long long *run[2], *keys[2];  // [tiles * CH_TILE] sorted tiles, the sorted list
+};
+
+// What the rewrite of the CSR reports back.
+struct RewriteOut {
+    unsigned long long edits[2];  // directed entries deleted, inserted
+    unsigned long long vnodes;    // of the new graph, as graph_finish counts them
+    unsigned int max_deg, err;
+};
+
+// Entries of one tile, in ascending order (bitonic in shared memory: 66 steps
+// of one exchange per thread, bound by their barriers; 17 us at any length up
+// to a wave of tiles).
+__global__ void __launch_bounds__(CH_TILE / 2) change_tiles(ChangeLists L, uint32_t n, RewriteOut *out) {
+    __shared__ unsigned long long key[CH_TILE];
+    const int w = blockIdx.x >= L.tiles[0];
+    const uint64_t t0 = (uint64_t)(blockIdx.x - (w ? L.tiles[0] : 0u)) * CH_TILE;
+    bool bad = false;
+    for (unsigned i = threadIdx.x; i < CH_TILE; i += blockDim.x) {
+        const uint64_t e = t0 + i;
+        unsigned long long k = ~0ull;
+        if (e < 2 * L.m[w]) {
+            const uint32_t u = L.src[w][e >> 1], v = L.dst[w][e >> 1];
+            if (u >= n || v >= n) bad = true;
+            else if (u != v) k = (e & 1) ? ((unsigned long long)v << 32 | u) : ((unsigned long long)u << 32 | v);
+        }
+        key[i] = k;
+    }
+    if (__syncthreads_or(bad) && threadIdx.x == 0) out->err = 1;
+    for (unsigned size = 2; size <= CH_TILE; size <<= 1)
+        for (unsigned stride = size >> 1; stride > 0; stride >>= 1) {
+            const unsigned i = 2 * threadIdx.x - (threadIdx.x & (stride - 1));
+            const unsigned long long x = key[i], y = key[i + stride];
+            if ((x > y) == ((i & size) == 0)) {
+                key[i] = y;
+                key[i + stride] = x;
             }
-            continue;
+            __syncthreads();
         }
-        const uint32_t *row = col + r0;
-        uint32_t wd = 0, wi = 0;
-        for (uint32_t b = 0; b < dl; b += 32) {
-            const uint32_t j = b + lane;
-            bool del = false;
-            uint32_t p = 0;
-            if (j < dl) {
-                const uint32_t x = dcol[d0 + j];
-                p = lower_bound_u32(row, len, x);
-                del = p < len && row[p] == x;
-                if (del && il) {
-                    const uint32_t q = lower_bound_u32(icol + i0, il, x);
-                    if (q < il && icol[i0 + q] == x) del = false;  // deleted and re-inserted: keep
-                }
+    for (unsigned i = threadIdx.x; i < CH_TILE; i += blockDim.x) L.run[w][t0 + i] = key[i];
+}
+
+// Merges the tiles: an entry's place in the list is its place in its own tile
+// plus its rank in every other one (equal entries keep the order of their
+// tiles).  The searches of different tiles do not depend on each other, so four
+// run at a time: 14 us for ten tiles.  Both kernels stand for the CSR build of
+// a change list, 125 us of passes over 4 M vertices.
+__global__ void __launch_bounds__(256) change_ranks(ChangeLists L) {
+    constexpr unsigned PER = CH_TILE / 256;
+    unsigned b = blockIdx.x;
+    const int w = b >= L.tiles[0] * PER;
+    if (w) b -= L.tiles[0] * PER;
+    const unsigned t = b / PER, tiles = L.tiles[w];
+    const unsigned i = (b % PER) * 256 + threadIdx.x;
+    const unsigned long long *run = L.run[w];
+    const unsigned long long x = run[(uint64_t)t * CH_TILE + i];
+    uint64_t rank = i;
+    constexpr int Q = 4;
+    for (unsigned o = 0; o < tiles; o += Q) {
+        unsigned pos[Q] = {};
+#pragma unroll
+        for (unsigned step = CH_TILE / 2; step > 0; step >>= 1)
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                if (o + q >= tiles) continue;
+                const unsigned long long y = __ldg(&run[(uint64_t)(o + q) * CH_TILE + pos[q] + step - 1]);
+                if (y < x || (y == x && o + q < t)) pos[q] += step;
             }
-            const unsigned m = __ballot_sync(KC_FULL_MASK, del);
-            if (del) dpos[d0 + wd + __popc(m & ((1u << lane) - 1u))] = p;
-            wd += __popc(m);
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            if (o + q >= tiles || o + q == t) continue;
+            const unsigned long long y = __ldg(&run[(uint64_t)(o + q) * CH_TILE + pos[q]]);  // pos <= CH_TILE - 1
+            rank += pos[q] + (y < x || (y == x && o + q < t) ? 1u : 0u);
         }
-        for (uint32_t b = 0; b < il; b += 32) {
-            const uint32_t j = b + lane;
-            bool ins = false;
-            uint32_t x = 0;
-            if (j < il) {
-                x = icol[i0 + j];
-                const uint32_t p = lower_bound_u32(row, len, x);
-                ins = !(p < len && row[p] == x);
-            }
-            const unsigned m = __ballot_sync(KC_FULL_MASK, ins);
-            if (ins) ival[i0 + wi + __popc(m & ((1u << lane) - 1u))] = x;
-            wi += __popc(m);
-        }
-        if (lane == 0) {
-            if (dcnt) dcnt[v] = wd;
-            if (icnt) icnt[v] = wi;
-            newlen[v] = len - wd + wi;
-        }
-        nd += wd;
-        ni += wi;
     }
-    if (lane == 0 && (nd || ni)) {
-        atomicAdd(&applied[0], nd);
-        atomicAdd(&applied[1], ni);
-    }
+    L.keys[w][rank] = x;
 }
 
-// Phase 2, one warp per row: write the merged, sorted row.
-// Runs of unchanged rows between consecutive changed rows: run j covers
-// rows changed[j-1]+1 .. changed[j]-1 (changed[-1] = -1, changed[R] = n);
-// its old entries [ra, rb) move by rd.
-__global__ void make_runs(const int64_t *__restrict__ rowptr, const int64_t *__restrict__ nrow,
-                          const uint32_t *__restrict__ changed, uint32_t R, uint32_t n, int64_t *ra, int64_t *rb,
-                          int64_t *rd) {
-    for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j <= R; j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t first = j ? changed[j - 1] + 1 : 0u;
-        const uint32_t end = j < R ? changed[j] : n;
-        ra[j] = rowptr[first];
-        rb[j] = rowptr[end > first ? end : first];
-        rd[j] = nrow[first] - rowptr[first];
-    }
-}
-
-// Bulk move of the unchanged rows: each CTA copies one tile of the old column
-// array, run by run (runs are ordered and usually span many tiles).
-constexpr uint64_t RUN_TILE = 8192;
-__global__ void copy_runs(const uint32_t *__restrict__ col, uint64_t nnz_old, const int64_t *__restrict__ ra,
-                          const int64_t *__restrict__ rb, const int64_t *__restrict__ rd, uint32_t R,
-                          uint32_t *ncol) {
-    for (uint64_t t0 = blockIdx.x * RUN_TILE; t0 < nnz_old; t0 += (uint64_t)gridDim.x * RUN_TILE) {
-        const uint64_t t1 = t0 + RUN_TILE < nnz_old ? t0 + RUN_TILE : nnz_old;
-        // first run ending after t0
-        uint32_t lo = 0, hi = R + 1;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if ((uint64_t)rb[mid] <= t0) lo = mid + 1;
-            else hi = mid;
-        }
-        for (uint32_t j = lo; j <= R && (uint64_t)ra[j] < t1; j++) {
-            const uint64_t a = (uint64_t)ra[j] > t0 ? (uint64_t)ra[j] : t0;
-            const uint64_t b = (uint64_t)rb[j] < t1 ? (uint64_t)rb[j] : t1;
-            const int64_t d = rd[j];
-            for (uint64_t e = a + threadIdx.x; e < b; e += blockDim.x) ncol[(int64_t)e + d] = col[e];
-        }
-    }
-}
-
-// The changed rows are written in chunks of MERGE_CHUNK old entries, one warp
-// per chunk, so a long row (deletions drawn from the edge set land on hub
-// rows of 10^5 entries) spreads over many warps instead of holding one warp
-// for the whole update.  nchunks[i] = chunks of changed row i (at least one,
-// so that a row that only gains entries still writes them).
-constexpr uint32_t MERGE_CHUNK = 1024;
-__global__ void merge_chunk_counts(const int64_t *__restrict__ rowptr, const uint32_t *__restrict__ changed,
-                                   uint32_t nchanged, uint32_t *nchunks) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nchanged;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = changed[i];
-        const uint64_t len = (uint64_t)(rowptr[v + 1] - rowptr[v]);
-        const uint64_t k = (len + MERGE_CHUNK - 1) / MERGE_CHUNK;
-        nchunks[i] = (uint32_t)(k > 0 ? k : 1);
-    }
-}
-
-// Chunk ci of the concatenated chunk lists (cstart: exclusive prefix of
-// nchunks, cstart[nchanged] = total): kept old entries p of its range move to
-// w0 + p - (deleted entries before p) + (inserted values below row[p]); the
-// row's inserted values are shared out over its chunks.
-__global__ void merge_write_chunks(const int64_t *__restrict__ rowptr, const uint32_t *__restrict__ col,
-                                   const uint32_t *__restrict__ changed, uint32_t nchanged,
-                                   const int64_t *__restrict__ cstart, uint64_t nch,
-                                   const int64_t *__restrict__ drp, const uint32_t *__restrict__ dpos,
-                                   const uint32_t *__restrict__ dcnt, const int64_t *__restrict__ irp,
-                                   const uint32_t *__restrict__ ival, const uint32_t *__restrict__ icnt,
-                                   const int64_t *__restrict__ nrow, uint32_t *ncol) {
+// The entries of a change list that the CSR builder sorted (one warp per 32
+// rows: most of them are empty).
+__global__ void list_keys(const int64_t *__restrict__ rowptr, const uint32_t *__restrict__ col, uint32_t n,
+                          unsigned long long *keys) {
     const unsigned lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t ci = warp; ci < nch; ci += nw) {
-        // changed row of this chunk: the last i with cstart[i] <= ci
-        uint32_t lo = 0, hi = nchanged;
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if ((uint64_t)cstart[mid] <= ci) lo = mid;
-            else hi = mid;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t v0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); v0 < n; v0 += stride) {
+        const uint64_t v = v0 + lane;
+        const int64_t a = v < n ? rowptr[v] : 0, z = v < n ? rowptr[v + 1] : 0;
+        unsigned rows = __ballot_sync(KC_FULL_MASK, z > a);
+        while (rows) {
+            const int l = __ffs(rows) - 1;
+            rows &= rows - 1;
+            const int64_t ra = __shfl_sync(KC_FULL_MASK, a, l), rz = __shfl_sync(KC_FULL_MASK, z, l);
+            for (int64_t e = ra + lane; e < rz; e += 32) keys[e] = (unsigned long long)(v0 + l) << 32 | col[e];
         }
-        const uint32_t v = changed[lo];
-        const uint32_t c = (uint32_t)(ci - (uint64_t)cstart[lo]);
-        const uint32_t nc = (uint32_t)(cstart[lo + 1] - cstart[lo]);
-        const int64_t r0 = rowptr[v];
-        const uint32_t len = (uint32_t)(rowptr[v + 1] - r0);
-        const int64_t w0 = nrow[v];
-        const uint32_t dc = dcnt ? dcnt[v] : 0u, ic = icnt ? icnt[v] : 0u;
-        const uint32_t *dp = dc ? dpos + drp[v] : nullptr;
-        const uint32_t *iv = ic ? ival + irp[v] : nullptr;
-        const uint32_t *row = col + r0;
-        const uint32_t p_end = min(len, (c + 1) * MERGE_CHUNK);
-        for (uint32_t p = c * MERGE_CHUNK + lane; p < p_end; p += 32) {
-            const uint32_t x = row[p];
-            const uint32_t before_d = dc ? lower_bound_u32(dp, dc, p) : 0u;
-            if (before_d < dc && dp[before_d] == p) continue;  // deleted
-            const uint32_t before_i = ic ? lower_bound_u32(iv, ic, x) : 0u;
-            ncol[w0 + p - before_d + before_i] = x;
+    }
+}
+
+// ------------------------------------------------------------- the rewrite ----
+// Sorted change lists turn into edits of the column array: positions of entries
+// that go, ascending, and positions before which an entry comes, ascending with
+// their keys.  The rewrite needs nothing per row: an old entry at e moves to
+// e - (deletions before e) + (insertions at or before e), and insertion k at
+// position p lands on p - (deletions before p) + k.
+struct Edits {
+    const unsigned long long *keys[2];
+    uint64_t len[2];
+    unsigned blocks[2];   // of 256 entries
+    int64_t *found[2];    // [len] position of every entry's edit, -1: none
+    uint32_t *count;      // [blocks[0] + blocks[1]] edits per block
+    const int64_t *base;  // prefix of count, or null: the few counts are added up where they are needed
+    int64_t *pos[2];      // the edits
+    unsigned long long *ikey;
+};
+
+// Which entries change the graph: a deletion that is in its row and not among
+// the insertions, an insertion that is not in its row; each once.
+__global__ void __launch_bounds__(256) plan_edits(const int64_t *__restrict__ rowptr, const uint32_t *__restrict__ col,
+                                                  Edits E) {
+    const int w = blockIdx.x >= E.blocks[0];
+    const uint64_t j = (uint64_t)(blockIdx.x - (w ? E.blocks[0] : 0u)) * 256 + threadIdx.x;
+    bool edit = false;
+    if (j < E.len[w]) {
+        const unsigned long long k = E.keys[w][j];
+        int64_t at = -1;
+        if (k != ~0ull && (j == 0 || E.keys[w][j - 1] != k)) {
+            const int64_t r0 = rowptr[k >> 32];
+            const uint64_t len = (uint64_t)(rowptr[(k >> 32) + 1] - r0);
+            const uint32_t x = (uint32_t)k;
+            const uint64_t p = count_below(col + r0, len, x);
+            const bool there = p < len && col[r0 + p] == x;
+            if (w) {
+                edit = !there;
+            } else if (there) {
+                const uint64_t q = count_below(E.keys[1], E.len[1], k);
+                edit = !(q < E.len[1] && E.keys[1][q] == k);  // deleted and inserted: it stays
+            }
+            if (edit) at = r0 + (int64_t)p;
         }
-        for (uint32_t j = c * 32 + lane; j < ic; j += nc * 32) {
-            const uint32_t y = iv[j];
-            const uint32_t lb = lower_bound_u32(row, len, y);
-            const uint32_t before_d = dc ? lower_bound_u32(dp, dc, lb) : 0u;
-            ncol[w0 + lb - before_d + j] = y;
+        E.found[w][j] = at;
+    }
+    const int c = __syncthreads_count(edit);
+    if (threadIdx.x == 0) E.count[blockIdx.x] = (uint32_t)c;
+}
+
+__global__ void __launch_bounds__(256) place_edits(Edits E, RewriteOut *out) {
+    __shared__ unsigned part[8];
+    __shared__ unsigned long long before;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int w = blockIdx.x >= E.blocks[0];
+    const unsigned first = w ? E.blocks[0] : 0u;
+    if (threadIdx.x == 0) before = E.base ? (unsigned long long)(E.base[blockIdx.x] - E.base[first]) : 0ull;
+    __syncthreads();
+    if (!E.base) {
+        unsigned s = 0;
+        for (unsigned b = first + threadIdx.x; b < blockIdx.x; b += 256) s += E.count[b];
+        s = __reduce_add_sync(KC_FULL_MASK, s);
+        if (lane == 0 && s) atomicAdd(&before, (unsigned long long)s);
+    }
+    const uint64_t j = (uint64_t)(blockIdx.x - first) * 256 + threadIdx.x;
+    const int64_t at = j < E.len[w] ? E.found[w][j] : -1;
+    const unsigned m = __ballot_sync(KC_FULL_MASK, at >= 0);
+    if (lane == 0) part[warp] = __popc(m);
+    __syncthreads();
+    unsigned long long o = before + __popc(m & ((1u << lane) - 1u));
+    for (unsigned i = 0; i < warp; i++) o += part[i];
+    if (at >= 0) {
+        E.pos[w][o] = at;
+        if (w) E.ikey[o] = E.keys[1][j];
+    }
+    if (threadIdx.x == 255 && blockIdx.x == first + E.blocks[w] - 1) out->edits[w] = o + (at >= 0 ? 1 : 0);
+}
+
+// New row offsets, and the new graph's largest degree and virtual-node count
+// from the same pass.  Each CTA looks up the edits of its rows once; a thread
+// searches them for its nine rows side by side (the hubs' tile holds most of
+// the edits, and one search after the other there outlasts the other tiles).
+constexpr unsigned ROW_TILE = 2048;
+__global__ void __launch_bounds__(256) shift_rows(const int64_t *__restrict__ rowptr, uint32_t n,
+                                                  const int64_t *__restrict__ dpos,
+                                                  const unsigned long long *__restrict__ ikey, RewriteOut *out,
+                                                  int64_t *nrow) {
+    __shared__ int64_t off[ROW_TILE + 1];
+    __shared__ uint64_t cut[4];
+    __shared__ unsigned long long vn_sum;
+    __shared__ unsigned md_max;
+    const uint64_t v0 = (uint64_t)blockIdx.x * ROW_TILE;
+    const uint64_t v1 = v0 + ROW_TILE < n ? v0 + ROW_TILE : n;
+    const unsigned rows = (unsigned)(v1 - v0);
+    constexpr unsigned PER = ROW_TILE / 256 + 1;
+    int64_t old[PER];  // on their way while the edits are looked up
+#pragma unroll
+    for (unsigned j = 0; j < PER; j++) {
+        const unsigned i = j * 256 + threadIdx.x;
+        if (i <= rows) old[j] = rowptr[v0 + i];
+    }
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < 4) {
+        const uint64_t v = warp & 1 ? v1 : v0;
+        const uint64_t c = warp < 2 ? warp_count_below(dpos, out->edits[0], rowptr[v])
+                                    : warp_count_below(ikey, out->edits[1], (unsigned long long)v << 32);
+        if (lane == 0) cut[warp] = c;
+    }
+    if (threadIdx.x == 128) {
+        vn_sum = 0;
+        md_max = 0;
+    }
+    __syncthreads();
+    const uint64_t d0 = cut[0], dn = cut[1] - d0, i0 = cut[2], in = cut[3] - i0;
+    uint64_t gone[PER] = {}, come[PER] = {};
+    for (uint64_t step = dn ? 1ull << (63 - __clzll((long long)dn)) : 0; step; step >>= 1)
+#pragma unroll
+        for (unsigned j = 0; j < PER; j++)
+            if (gone[j] + step <= dn && j * 256 + threadIdx.x <= rows && __ldg(&dpos[d0 + gone[j] + step - 1]) < old[j])
+                gone[j] += step;
+    for (uint64_t step = in ? 1ull << (63 - __clzll((long long)in)) : 0; step; step >>= 1)
+#pragma unroll
+        for (unsigned j = 0; j < PER; j++)
+            if (come[j] + step <= in && (__ldg(&ikey[i0 + come[j] + step - 1]) >> 32) < v0 + j * 256 + threadIdx.x)
+                come[j] += step;
+#pragma unroll
+    for (unsigned j = 0; j < PER; j++) {
+        const unsigned i = j * 256 + threadIdx.x;
+        if (i > rows) continue;
+        off[i] = old[j] - (int64_t)(d0 + gone[j]) + (int64_t)(i0 + come[j]);
+        if (i < rows || v1 == n) nrow[v0 + i] = off[i];
+    }
+    __syncthreads();
+    unsigned md = 0;
+    unsigned long long vn = 0;
+    for (unsigned i = threadIdx.x; i < rows; i += 256) {
+        const uint64_t d = (uint64_t)(off[i + 1] - off[i]);
+        md = max(md, (unsigned)d);
+        vn += (d + 31) / 32;
+    }
+    md = __reduce_max_sync(KC_FULL_MASK, md);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) vn += __shfl_xor_sync(KC_FULL_MASK, vn, o);
+    if (lane == 0) {
+        atomicMax(&md_max, md);
+        atomicAdd(&vn_sum, vn);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMax(&out->max_deg, md_max);
+        atomicAdd(&out->vnodes, vn_sum);
+    }
+}
+
+// The new column array.  A CTA takes a tile of old entries and looks up the
+// edits in it; its warps narrow them to chunks of 512 entries, and a chunk
+// without edits (with 10^4 edges on 128 M entries all but one in seven) is a
+// plain copy with sixteen loads in flight per lane.  Bound by memory: the two
+// arrays do not share alignment, so accesses stay 4 bytes wide per lane and the
+// rate comes from 40 warps per SM: 128 M entries with 20,000 edits in 165 us
+// (6.2 TB/s; 172 us with four CTAs per SM, 202 us with the tile's edits looked
+// up by one thread each).  Runs of unchanged rows copied apart from the changed
+// rows, which warps merged entry by entry, took 260 + 95 us.
+constexpr uint64_t MOVE_TILE = 8192;
+constexpr unsigned MOVE_CHUNK = 512;
+__global__ void __launch_bounds__(256, 5) move_entries(const uint32_t *__restrict__ col, uint64_t nnz,
+                                                    const int64_t *__restrict__ dpos, const int64_t *__restrict__ ipos,
+                                                    const unsigned long long *__restrict__ ikey,
+                                                    const RewriteOut *__restrict__ out, uint32_t *ncol) {
+    __shared__ uint64_t cut[4];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t t0 = (uint64_t)blockIdx.x * MOVE_TILE;
+    const bool last = t0 + MOVE_TILE >= nnz;
+    const uint64_t t1 = last ? nnz : t0 + MOVE_TILE;
+    if (warp < 4) {
+        const uint64_t len = out->edits[warp >> 1];
+        const uint64_t c = warp == 3 && last ? len  // those behind the last entry too
+                                             : warp_count_below(warp < 2 ? dpos : ipos, len, (int64_t)(warp & 1 ? t1 : t0));
+        if (lane == 0) cut[warp] = c;
+    }
+    __syncthreads();
+    const uint64_t d0 = cut[0], d1 = cut[1], i0 = cut[2], i1 = cut[3];
+    for (uint64_t k = i0 + threadIdx.x; k < i1; k += 256) {
+        const int64_t p = ipos[k];
+        ncol[(uint64_t)p - d0 - count_below(dpos + d0, d1 - d0, p) + k] = (uint32_t)ikey[k];
+    }
+    for (uint64_t c = t0 + warp * MOVE_CHUNK; c < t1; c += 8 * MOVE_CHUNK) {
+        const uint64_t ce = c + MOVE_CHUNK < t1 ? c + MOVE_CHUNK : t1;
+        const uint64_t a = d0 + count_below(dpos + d0, d1 - d0, (int64_t)c);
+        const uint64_t an = d0 + count_below(dpos + d0, d1 - d0, (int64_t)ce) - a;
+        const uint64_t b = i0 + count_below(ipos + i0, i1 - i0, (int64_t)c);
+        const uint64_t bn = i0 + count_below(ipos + i0, i1 - i0, (int64_t)ce) - b;
+        uint32_t x[MOVE_CHUNK / 32];
+#pragma unroll
+        for (unsigned i = 0; i < MOVE_CHUNK / 32; i++) {
+            const uint64_t e = c + i * 32 + lane;
+            if (e < ce) x[i] = __ldcs(&col[e]);
+        }
+        if (an == 0 && bn == 0) {
+#pragma unroll
+            for (unsigned i = 0; i < MOVE_CHUNK / 32; i++) {
+                const uint64_t e = c + i * 32 + lane;
+                if (e < ce) ncol[e - a + b] = x[i];
+            }
+        } else {
+#pragma unroll
+            for (unsigned i = 0; i < MOVE_CHUNK / 32; i++) {
+                const uint64_t e = c + i * 32 + lane;
+                if (e >= ce) continue;
+                const uint64_t g = count_below(dpos + a, an, (int64_t)e);
+                if (g < an && dpos[a + g] == (int64_t)e) continue;
+                ncol[e - a - g + b + count_below(ipos + b, bn, (int64_t)e + 1)] = x[i];
+            }
         }
     }
 }
@@ -369,121 +518,120 @@ struct Scratch {
 
 // Rewrites g's CSR: minus the edges of `del`, plus the edges of `ins` (both
 // undirected edge lists on the device; either may be empty).  Counts the
-// undirected edges actually deleted / inserted.
+// undirected edges actually deleted / inserted.  The graph stays as it was
+// until the rewrite is known to have succeeded; the host waits once, at its end.
 static int apply_changes(Graph *g, const uint32_t *d_isrc, const uint32_t *d_idst, uint64_t mi, const uint32_t *d_dsrc,
                          const uint32_t *d_ddst, uint64_t md, uint64_t *n_del, uint64_t *n_ins) {
     cudaStream_t s = g->stream;
     const uint32_t n = g->n;
-    Graph dg, ig;  // per-row change lists, built like any graph
-    dg.device = ig.device = g->device;
-    dg.sm_count = ig.sm_count = g->sm_count;
-    // the temporaries borrow g's stream only while they are built (their
-    // destructor would otherwise destroy it)
-    if (md) {
-        dg.stream = s;
-        const int rc = build_csr_from_edges(&dg, d_dsrc, d_ddst, md, n, KC_EDGES_DEDUP);
-        dg.stream = nullptr;
+    const uint64_t m[2] = {md, mi};
+    const uint32_t *src[2] = {d_dsrc, d_isrc}, *dst[2] = {d_ddst, d_idst};
+    // long lists: sorted by the builder, like any graph
+    Graph lists[2];
+    ChangeLists L{};
+    Edits E{};
+    for (int w = 0; w < 2; w++) {
+        E.len[w] = 2 * m[w];
+        if (2 * m[w] <= CH_TILED_MAX) {
+            L.src[w] = src[w];
+            L.dst[w] = dst[w];
+            L.m[w] = m[w];
+            L.tiles[w] = (unsigned)((2 * m[w] + CH_TILE - 1) / CH_TILE);
+            continue;
+        }
+        Graph &q = lists[w];
+        q.device = g->device;
+        q.sm_count = g->sm_count;
+        // borrows g's stream only while it is built (its destructor would
+        // otherwise destroy it)
+        q.stream = s;
+        const int rc = build_csr_from_edges(&q, src[w], dst[w], m[w], n, KC_EDGES_DEDUP);
+        q.stream = nullptr;
         if (rc) return rc;
+        E.len[w] = q.nnz;
     }
-    if (mi) {
-        ig.stream = s;
-        const int rc = build_csr_from_edges(&ig, d_isrc, d_idst, mi, n, KC_EDGES_DEDUP);
-        ig.stream = nullptr;
-        if (rc) return rc;
+    for (int w = 0; w < 2; w++) E.blocks[w] = (unsigned)((E.len[w] + 255) / 256);
+    const unsigned blocks = E.blocks[0] + E.blocks[1];
+    // one allocation for everything of the lists' size: the report, per list
+    // the sorted tiles (later the edits found), the keys and the edits, the
+    // counts and their prefix
+    uint64_t cap[2], words = sizeof(RewriteOut) / 8;
+    for (int w = 0; w < 2; w++) {
+        cap[w] = std::max<uint64_t>((uint64_t)L.tiles[w] * CH_TILE, E.len[w]);
+        words += 3 * cap[w];
     }
+    words += cap[1] + ((uint64_t)blocks + 1) / 2 + blocks + 2;
     Scratch sc;
     sc.stream = s;
-    uint32_t *dpos = nullptr, *dcnt = nullptr, *ival = nullptr, *icnt = nullptr, *newlen = nullptr;
-    unsigned long long *applied = nullptr;
-    if (md) {
-        KC_TRY(sc.get(&dpos, dg.nnz, "deleted positions"));
-        KC_TRY(sc.get(&dcnt, n, "deleted counts"));
+    unsigned long long *w8 = nullptr;
+    KC_TRY(sc.get(&w8, words, "change lists"));
+    RewriteOut *out = reinterpret_cast<RewriteOut *>(w8);
+    unsigned long long *next = w8 + sizeof(RewriteOut) / 8;
+    for (int w = 0; w < 2; w++) {
+        L.run[w] = next;
+        L.keys[w] = next + cap[w];
+        E.keys[w] = L.keys[w];
+        E.found[w] = reinterpret_cast<int64_t *>(L.run[w]);
+        E.pos[w] = reinterpret_cast<int64_t *>(next + 2 * cap[w]);
+        next += 3 * cap[w];
     }
-    if (mi) {
-        KC_TRY(sc.get(&ival, ig.nnz, "inserted values"));
-        KC_TRY(sc.get(&icnt, n, "inserted counts"));
+    E.ikey = next;
+    next += cap[1];
+    int64_t *base = reinterpret_cast<int64_t *>(next);
+    next += blocks + 1;
+    E.count = reinterpret_cast<uint32_t *>(next);
+    KC_CUDA(cudaMemsetAsync(out, 0, sizeof(RewriteOut), s));
+    const unsigned tiles = L.tiles[0] + L.tiles[1];
+    if (tiles) {
+        change_tiles<<<tiles, CH_TILE / 2, 0, s>>>(L, n, out);
+        change_ranks<<<tiles * (CH_TILE / 256), 256, 0, s>>>(L);
     }
-    KC_TRY(sc.get(&newlen, n, "new row lengths"));
-    KC_TRY(sc.get(&applied, 2, "applied counts"));
-    uint32_t *flag = nullptr;
-    int64_t *cpos = nullptr;
-    KC_TRY(sc.get(&flag, n, "changed-row flags"));
-    KC_TRY(sc.get(&cpos, (uint64_t)n + 1, "changed-row positions"));
-    KC_CUDA(cudaMemsetAsync(applied, 0, 16, s));
-    const int64_t *drp = md ? dg.rowptr : nullptr, *irp = mi ? ig.rowptr : nullptr;
-    // only the rows that the change lists touch are planned and rewritten
-    // row by row; the others move as whole runs
-    mark_changed<<<grid_of(g, n), 256, 0, s>>>(g->rowptr, n, drp, irp, dcnt, icnt, newlen, flag);
-    KC_TRY(exclusive_scan_u32_i64(flag, cpos, n, s));
-    int64_t R64 = 0;
-    KC_CUDA(cudaMemcpyAsync(&R64, cpos + n, 8, cudaMemcpyDeviceToHost, s));
-    KC_CUDA(cudaStreamSynchronize(s));
-    const uint32_t R = (uint32_t)R64;
-    uint32_t *changed = nullptr;
-    int64_t *ra = nullptr, *rb = nullptr, *rd = nullptr;
-    KC_TRY(sc.get(&changed, (uint64_t)R + 1, "changed rows"));
-    KC_TRY(sc.get(&ra, (uint64_t)R + 1, "run starts"));
-    KC_TRY(sc.get(&rb, (uint64_t)R + 1, "run ends"));
-    KC_TRY(sc.get(&rd, (uint64_t)R + 1, "run shifts"));
-    list_changed<<<grid_of(g, n), 256, 0, s>>>(flag, cpos, n, changed);
-    const int gw = grid_of(g, (uint64_t)std::max<uint32_t>(R, 1) * 32);
-    if (R)
-        merge_plan<<<gw, 256, 0, s>>>(g->rowptr, g->col, changed, R, drp, md ? dg.col : nullptr, irp,
-                                      mi ? ig.col : nullptr, dpos, dcnt, ival, icnt, newlen, applied);
-    // chunks of the changed rows for the merge
-    uint32_t *nchunks = nullptr;
-    int64_t *cstart = nullptr;
-    KC_TRY(sc.get(&nchunks, (uint64_t)R + 1, "merge chunk counts"));
-    KC_TRY(sc.get(&cstart, (uint64_t)R + 1, "merge chunk starts"));
-    if (R) {
-        merge_chunk_counts<<<grid_of(g, R), 256, 0, s>>>(g->rowptr, changed, R, nchunks);
-        KC_TRY(exclusive_scan_u32_i64(nchunks, cstart, R, s));
+    for (int w = 0; w < 2; w++)
+        if (lists[w].nnz)
+            list_keys<<<grid_of(g, n), 256, 0, s>>>(lists[w].rowptr, lists[w].col, n, L.keys[w]);
+    if (blocks) {
+        plan_edits<<<blocks, 256, 0, s>>>(g->rowptr, g->col, E);
+        if (blocks > 2 * CH_TILED_MAX / 256) {
+            KC_TRY(exclusive_scan_u32_i64(E.count, base, blocks, s));
+            E.base = base;
+        }
+        place_edits<<<blocks, 256, 0, s>>>(E, out);
     }
     int64_t *rp_new = nullptr;
+    uint32_t *col_new = nullptr;
     KC_TRY(dalloc(&rp_new, (uint64_t)n + 1, "row offsets"));
-    int rc = exclusive_scan_u32_i64(newlen, rp_new, n, s);
-    int64_t nnz_new = 0, nch = 0;
-    if (!rc) {
-        cudaMemcpyAsync(&nnz_new, rp_new + n, 8, cudaMemcpyDeviceToHost, s);
-        if (R) cudaMemcpyAsync(&nch, cstart + R, 8, cudaMemcpyDeviceToHost, s);
-        cudaError_t e0 = cudaStreamSynchronize(s);
-        if (e0 != cudaSuccess) rc = fail(KC_ERR_CUDA, "CSR merge plan: %s", cudaGetErrorString(e0));
+    int rc = dalloc(&col_new, g->nnz + E.len[1] + 1, "column ids");
+    if (rc) {
+        cudaStreamSynchronize(s);
+        dfree(rp_new);
+        return rc;
     }
-    if (!rc) {
-        uint32_t *col_new = nullptr;
-        rc = dalloc(&col_new, (uint64_t)nnz_new + 1, "column ids");
-        if (!rc) {
-            make_runs<<<grid_of(g, (uint64_t)R + 1), 256, 0, s>>>(g->rowptr, rp_new, changed, R, n, ra, rb, rd);
-            if (g->nnz) {
-                const uint64_t tiles = (g->nnz + RUN_TILE - 1) / RUN_TILE;
-                const int cb = (int)std::min<uint64_t>(tiles, (uint64_t)g->sm_count * 16);
-                copy_runs<<<cb, 256, 0, s>>>(g->col, g->nnz, ra, rb, rd, R, col_new);
-            }
-            if (R && nch > 0)
-                merge_write_chunks<<<grid_of(g, (uint64_t)nch * 32), 256, 0, s>>>(
-                    g->rowptr, g->col, changed, R, cstart, (uint64_t)nch, drp, dpos, dcnt, irp, ival, icnt, rp_new,
-                    col_new);
-            unsigned long long h[2];
-            cudaMemcpyAsync(h, applied, 16, cudaMemcpyDeviceToHost, s);
-            cudaError_t e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) {
-                dfree(col_new);
-                rc = fail(KC_ERR_CUDA, "CSR merge: %s", cudaGetErrorString(e));
-            } else {
-                dfree(g->rowptr);
-                dfree(g->col);
-                g->rowptr = rp_new;
-                g->col = col_new;
-                g->nnz = (uint64_t)nnz_new;
-                rp_new = nullptr;
-                *n_del = h[0] / 2;
-                *n_ins = h[1] / 2;
-            }
-        }
+    shift_rows<<<(unsigned)(((uint64_t)n + ROW_TILE - 1) / ROW_TILE + (n == 0)), 256, 0, s>>>(
+        g->rowptr, n, E.pos[0], E.ikey, out, rp_new);
+    move_entries<<<(unsigned)((g->nnz + MOVE_TILE - 1) / MOVE_TILE + (g->nnz == 0)), 256, 0, s>>>(
+        g->col, g->nnz, E.pos[0], E.pos[1], E.ikey, out, col_new);
+    RewriteOut h{};
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, out, sizeof(h), cudaMemcpyDeviceToHost, s);
+    const cudaError_t es = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = es;
+    if (e != cudaSuccess) rc = fail(KC_ERR_CUDA, "CSR merge: %s", cudaGetErrorString(e));
+    else if (h.err) rc = fail(KC_ERR_INVALID, "edge endpoint >= n (%u)", n);
+    if (rc) {
+        dfree(rp_new);
+        dfree(col_new);
+        return rc;
     }
-    dfree(rp_new);
-    if (rc) return rc;
-    return graph_finish(g);
+    dfree(g->rowptr);
+    dfree(g->col);
+    g->rowptr = rp_new;
+    g->col = col_new;
+    g->nnz = g->nnz - h.edits[0] + h.edits[1];
+    g->max_deg = h.max_deg;
+    g->num_vnodes = h.vnodes;
+    *n_del = h.edits[0] / 2;
+    *n_ins = h.edits[1] / 2;
+    return KC_OK;
 }
 
 static int ensure_maint(Graph *g) {
