@@ -87,6 +87,7 @@ struct PeelCtl {
     unsigned int levels;             // non-empty levels
     unsigned int kmax;               // largest level with a claim
     unsigned int zeros;              // degree-0 vertices (level 0)
+    unsigned int first;              // first level above 0 (the smallest degree above 0)
     PeelDone done[3];
     PeelQueue q[3][PEEL_MAX_QUEUES]; // shared spill queues of level i (slot i % 3)
 };

@@ -140,6 +140,7 @@ __global__ void peel_ctl_reset(PeelCtl *ctl, unsigned int grid) {
     }
     if (t == 0) {
         ctl->zeros = 0;
+        ctl->first = NO_LEVEL;
         ctl->err = 0;
         ctl->err_info = 0;
         ctl->level_indices = 0;
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
     }
     if (blockIdx.x == 0 && tid == 0) {
         if (ld_relaxed(&ctl->zeros)) ctl->levels = 1;
+        ctl->first = level_sh;
         if (A.trace && A.trace_cap) {
             A.trace[0].t_start_ns = global_ns();
             A.trace[0].level = 0;
@@ -1044,6 +1046,7 @@ int peel_run(Graph *g, cudaStream_t s, bool gpp_zero_to_one_flag, kc_stats *st) 
         st->iterations = h.level_indices;
         st->levels = h.levels;
         st->kmax = h.kmax;
+        st->kmin = h.zeros ? 0u : std::min(10u, h.first);
         st->ms = ms;
     }
     return KC_OK;
