@@ -48,9 +48,16 @@
 //     vertices leave a warp 32 at a time (Erdos-Renyi 10^6 / 8 x 10^6 1.94 ->
 //     1.20 ms, R-MAT 18 1.86 -> 1.35, R-MAT 22 7.45 -> 7.41, R-MAT 25 with a
 //     planted core 72.6 -> 67.2);
-//   * updates are visible at once within a sweep (Gauss-Seidel), which only
-//     shortens the trajectory; sweeps are separated by a grid barrier with a
-//     bounded wait.
+//   * an update may be seen at once within a sweep (Gauss-Seidel), which only
+//     shortens the trajectory, or from the next sweep on: the rule above holds
+//     for neighbours' estimates as old as the sweep's start, so these (and the
+//     pending bits, which only get set during a sweep) are read through the L1,
+//     which every SM drops at the grid barrier between sweeps.  Hubs are gathered
+//     by all SMs at a time, and from the L1 they neither queue at their L2 slice
+//     nor take its latency: R-MAT 18 1.35 -> 1.24 ms, R-MAT 22 7.45 -> 6.32,
+//     R-MAT 25 with a planted core 67.2 -> 64.2; without hubs nothing is gained
+//     (Erdos-Renyi 10^6 / 8 x 10^6 1.18 -> 1.20).  The waits of the barrier are
+//     bounded.
 #include <algorithm>
 
 #include "kc_device.cuh"
@@ -343,7 +350,7 @@ __device__ __forceinline__ void hx_activate_all(const HxArgs &A, const uint32_t 
     bool need[K];
 #pragma unroll
     for (int k = 0; k < K; k++)
-        need[k] = cand[k] && !(__ldcg(&A.inlist[nxt][u[k] >> 5]) & (1u << (u[k] & 31)));
+        need[k] = cand[k] && !(A.inlist[nxt][u[k] >> 5] & (1u << (u[k] & 31)));
     unsigned old[K];
 #pragma unroll
     for (int k = 0; k < K; k++) old[k] = need[k] ? atomicOr(&A.inlist[nxt][u[k] >> 5], 1u << (u[k] & 31)) : ~0u;
@@ -445,7 +452,7 @@ __device__ __forceinline__ uint32_t hx_warp_lower(const HxRow &R, const uint32_t
         __syncwarp();
         const int64_t ee = R.end(lo);
         for (int64_t j = R.s + lane; j < ee; j += 32) {
-            const uint32_t x = __ldcg(&c[R.r[j]]);
+            const uint32_t x = c[R.r[j]];
             if (x < hi && x >= lo) atomicAdd(&hist[x - lo], 1u);
         }
         __syncwarp();
@@ -471,7 +478,7 @@ __device__ __forceinline__ uint32_t hx_warp_gather(const uint32_t *row, const ui
         }
         uint32_t xx[HX_STREAM];
 #pragma unroll
-        for (int k = 0; k < HX_STREAM; k++) xx[k] = uu[k] != 0xffffffffu ? __ldcg(&c[uu[k]]) : 0u;
+        for (int k = 0; k < HX_STREAM; k++) xx[k] = uu[k] != 0xffffffffu ? c[uu[k]] : 0u;
 #pragma unroll
         for (int k = 0; k < HX_STREAM; k++)
             if (uu[k] != 0xffffffffu) {
@@ -535,7 +542,7 @@ __device__ bool hx_warp_vertex(const HxArgs &A, const HxVertex &x, unsigned cur,
             cu[k] = j < e ? A.col[j] : 0xffffffffu;
         }
 #pragma unroll
-        for (int k = 0; k < HX_CACHE; k++) cv[k] = cu[k] != 0xffffffffu ? __ldcg(&A.c[cu[k]]) : 0u;
+        for (int k = 0; k < HX_CACHE; k++) cv[k] = cu[k] != 0xffffffffu ? A.c[cu[k]] : 0u;
 #pragma unroll
         for (int k = 0; k < HX_CACHE; k++) cnt += (cu[k] != 0xffffffffu && cv[k] >= cap) ? 1u : 0u;
         cnt = __reduce_add_sync(KC_FULL_MASK, cnt);
@@ -631,7 +638,7 @@ __device__ bool hx_warp_vertex(const HxArgs &A, const HxVertex &x, unsigned cur,
                 uu[k] = j < en ? R.r[j] : 0xffffffffu;
             }
 #pragma unroll
-            for (int k = 0; k < HX_STREAM; k++) xx[k] = uu[k] != 0xffffffffu ? __ldcg(&A.c[uu[k]]) : 0u;
+            for (int k = 0; k < HX_STREAM; k++) xx[k] = uu[k] != 0xffffffffu ? A.c[uu[k]] : 0u;
             bool cand[HX_STREAM];
 #pragma unroll
             for (int k = 0; k < HX_STREAM; k++) cand[k] = uu[k] != 0xffffffffu && xx[k] > h && xx[k] <= cap;
@@ -662,7 +669,7 @@ __device__ unsigned hx_warp_tiny(const HxArgs &A, const HxVertex &x, bool valid,
         cu[k] = valid && j < e ? A.col[j] : 0xffffffffu;
     }
 #pragma unroll
-    for (int k = 0; k < 4; k++) cv[k] = cu[k] != 0xffffffffu ? __ldcg(&A.c[cu[k]]) : 0u;
+    for (int k = 0; k < 4; k++) cv[k] = cu[k] != 0xffffffffu ? A.c[cu[k]] : 0u;
     uint32_t cnt = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) cnt += (cu[k] != 0xffffffffu && cv[k] >= cap) ? 1u : 0u;
@@ -835,7 +842,7 @@ __device__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint3
                 uu[k] = j < j1 ? row[j] : 0xffffffffu;
             }
 #pragma unroll
-            for (int k = 0; k < HX_CACHE; k++) xx[k] = uu[k] != 0xffffffffu ? __ldcg(&A.c[uu[k]]) : 0u;
+            for (int k = 0; k < HX_CACHE; k++) xx[k] = uu[k] != 0xffffffffu ? A.c[uu[k]] : 0u;
 #pragma unroll
             for (int k = 0; k < HX_CACHE; k++)
                 if (uu[k] != 0xffffffffu) {
@@ -874,7 +881,7 @@ __device__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint3
                     uu[k] = j < j1 ? row[j] : 0xffffffffu;
                 }
 #pragma unroll
-                for (int k = 0; k < HX_CACHE; k++) xx[k] = uu[k] != 0xffffffffu ? __ldcg(&A.c[uu[k]]) : 0u;
+                for (int k = 0; k < HX_CACHE; k++) xx[k] = uu[k] != 0xffffffffu ? A.c[uu[k]] : 0u;
 #pragma unroll
                 for (int k = 0; k < HX_CACHE; k++)
                     if (uu[k] != 0xffffffffu && xx[k] < capw) atomicAdd(&hist[xx[k]], 1u);
@@ -895,7 +902,7 @@ __device__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint3
             uint32_t above = 0;
             const int64_t ee = upto((uint32_t)lo);
             for (int64_t j = s + threadIdx.x; j < ee; j += HX_THREADS) {
-                uint32_t x = __ldcg(&A.c[row[j]]);
+                uint32_t x = A.c[row[j]];
                 if (x >= hi) above++;
                 else if (x >= lo) atomicAdd(&hist[(x - lo) / w], 1u);
             }
@@ -932,7 +939,7 @@ __device__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint3
                 uu[k] = j < en ? row[j] : 0xffffffffu;
             }
 #pragma unroll
-            for (int k = 0; k < HX_CACHE; k++) xx[k] = uu[k] != 0xffffffffu ? __ldcg(&A.c[uu[k]]) : 0u;
+            for (int k = 0; k < HX_CACHE; k++) xx[k] = uu[k] != 0xffffffffu ? A.c[uu[k]] : 0u;
             bool cand[HX_CACHE];
 #pragma unroll
             for (int k = 0; k < HX_CACHE; k++) cand[k] = uu[k] != 0xffffffffu && xx[k] > h && xx[k] <= cap;
