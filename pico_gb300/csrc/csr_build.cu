@@ -197,15 +197,22 @@ __global__ void scatter_edges(const uint32_t *__restrict__ src, const uint32_t *
 //   part_pairs   (row, column) pairs grouped by bucket: a tile of edges is
 //                grouped in shared memory and written out bucket by bucket;
 //   part_degrees row counts of every tile, added to the degrees (one atomic per
-//                row of a tile; a bucket of one tile writes them);
-//   part_rows    every tile reserves its share of each row, then places its
-//                columns at shared-memory cursors.
-// What bounds it is memory: the pairs are written once and read three times.
-// R-MAT 22 (134 M entries): 0.12 + 0.86 + 0.19 + 1.16 ms and 0.03 ms of scans,
+//                row of a tile; a bucket of one tile writes them), and where in
+//                its row each tile's share begins;
+//   part_rows    every tile sorts its columns by row in shared memory and writes
+//                them out row by row.
+// What bounds it is memory and the shared-memory atomics: the pairs are written
+// once and read twice, each time with one atomic per entry (6 G/s per SM).
+// R-MAT 22 (134 M entries): 0.12 + 0.62 + 0.21 + 0.60 ms and 0.03 ms of scans,
 // where counting and scattering took 5.05 ms.
 constexpr int PART_THREADS = 512;
-constexpr int PART_PER = 8;                                // edges per thread of part_pairs
-constexpr uint32_t PART_EDGES = PART_THREADS * PART_PER;   // edges it groups at a time
+// part_pairs groups 8,192 edges at a time: 8 pairs (two sectors) per bucket on
+// average with 2,048 buckets, one CTA per SM.  Half as many edges, two CTAs per
+// SM: whole builds of R-MAT 22 4.25 ms instead of 4.13, of a uniform random
+// graph of 10^6 vertices and 16 M edges 1.15 instead of 1.05.
+constexpr int PAIR_THREADS = 1024;
+constexpr int PART_PER = 8;                                // edges per thread
+constexpr uint32_t PART_EDGES = PAIR_THREADS * PART_PER;
 constexpr uint32_t PART_TILE = 32768;                      // entries per tile of a bucket
 constexpr uint32_t PART_MAX_BUCKETS = 4096;
 constexpr int PART_MAX_SHIFT = 14;                         // 64 KB of row counters
@@ -214,6 +221,8 @@ struct PartPlan {
     uint64_t *base;    // [buckets + 1] first pair of each bucket
     uint64_t *cursor;  // [buckets]     next free pair while partitioning
     uint32_t *tile;    // [buckets + 1] first tile of each bucket
+    uint32_t *off;     // [tiles << shift] where each tile's share of a row begins (unset where it has none)
+    uint16_t *count;   // [tiles << shift] and how long it is (a tile has 32,768 entries)
     uint32_t buckets;
     int shift;
 };
@@ -280,27 +289,27 @@ __global__ void __launch_bounds__(1024) part_plan(PartPlan plan) {
 
 // Shared memory: pairs of a tile, then per bucket the distance from a pair's
 // place in the tile to its place in the output, and the bucket's count.
-__global__ void __launch_bounds__(PART_THREADS) part_pairs(const uint32_t *__restrict__ src,
+__global__ void __launch_bounds__(PAIR_THREADS) part_pairs(const uint32_t *__restrict__ src,
                                                            const uint32_t *__restrict__ dst, uint64_t m, uint32_t n,
                                                            PartPlan plan, uint2 *pairs) {
     extern __shared__ __align__(16) unsigned char part_sm[];
     uint2 *stage = reinterpret_cast<uint2 *>(part_sm);
     unsigned long long *delta = reinterpret_cast<unsigned long long *>(stage + 2 * PART_EDGES);
     uint32_t *cnt = reinterpret_cast<uint32_t *>(delta + plan.buckets);
-    __shared__ uint32_t wsum[PART_THREADS / 32];
+    __shared__ uint32_t wsum[PAIR_THREADS / 32];
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t per = (plan.buckets + PART_THREADS - 1) / PART_THREADS;
+    const uint32_t per = (plan.buckets + PAIR_THREADS - 1) / PAIR_THREADS;
     for (uint64_t t0 = (uint64_t)blockIdx.x * PART_EDGES; t0 < m; t0 += (uint64_t)gridDim.x * PART_EDGES) {
-        for (uint32_t b = threadIdx.x; b < plan.buckets; b += PART_THREADS) cnt[b] = 0;
+        for (uint32_t b = threadIdx.x; b < plan.buckets; b += PAIR_THREADS) cnt[b] = 0;
         uint32_t a[PART_PER], b[PART_PER];
 #pragma unroll
         for (int k = 0; k < PART_PER; k++) {
-            const uint64_t i = t0 + (uint64_t)k * PART_THREADS + threadIdx.x;
+            const uint64_t i = t0 + (uint64_t)k * PAIR_THREADS + threadIdx.x;
             a[k] = i < m ? src[i] : 0u;
             b[k] = i < m ? dst[i] : 0u;
         }
         __syncthreads();
-        uint32_t rank[PART_PER];  // of both directions, 16 bits each (a tile has 8,192 pairs)
+        uint32_t rank[PART_PER];  // of both directions, 16 bits each (a tile has 16,384 pairs)
 #pragma unroll
         for (int k = 0; k < PART_PER; k++) {
             rank[k] = 0;
@@ -314,7 +323,7 @@ __global__ void __launch_bounds__(PART_THREADS) part_pairs(const uint32_t *__res
         __syncthreads();
         // exclusive prefix of the counts; each bucket's pairs are reserved in
         // the output with one atomic
-        constexpr uint32_t PER = PART_MAX_BUCKETS / PART_THREADS;
+        constexpr uint32_t PER = PART_MAX_BUCKETS / PAIR_THREADS;
         const uint32_t b0 = threadIdx.x * per;
         uint32_t c[PER], own = 0;
         unsigned long long to[PER];
@@ -330,7 +339,7 @@ __global__ void __launch_bounds__(PART_THREADS) part_pairs(const uint32_t *__res
         uint32_t at = warp_excl_scan(own, lane, wtot);
         if (lane == 0) wsum[warp] = wtot;
         __syncthreads();
-        const uint32_t ws = lane < PART_THREADS / 32 ? wsum[lane] : 0u;
+        const uint32_t ws = lane < PAIR_THREADS / 32 ? wsum[lane] : 0u;
         at += __reduce_add_sync(KC_FULL_MASK, lane < warp ? ws : 0u);
         const uint32_t total = __reduce_add_sync(KC_FULL_MASK, ws);
 #pragma unroll
@@ -348,7 +357,7 @@ __global__ void __launch_bounds__(PART_THREADS) part_pairs(const uint32_t *__res
                 stage[cnt[b[k] >> plan.shift] + (rank[k] >> 16)] = make_uint2(b[k], a[k]);
             }
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < total; i += PART_THREADS) {
+        for (uint32_t i = threadIdx.x; i < total; i += PAIR_THREADS) {
             const uint2 q = stage[i];
             pairs[delta[q.x >> plan.shift] + i] = q;
         }
@@ -386,40 +395,88 @@ __global__ void __launch_bounds__(PART_THREADS) part_degrees(const uint2 *__rest
         const uint64_t r0 = (uint64_t)b << plan.shift;
         for (uint32_t i = threadIdx.x; i < rows && r0 + i < n; i += PART_THREADS) {
             const uint32_t c = rows_sm[i];
+            const uint64_t at = ((uint64_t)t << plan.shift) + i;
+            plan.count[at] = (uint16_t)c;
             if (!c) continue;
             if (alone) deg[r0 + i] = c;
-            else atomicAdd(&deg[r0 + i], c);
+            plan.off[at] = alone ? 0u : atomicAdd(&deg[r0 + i], c);
         }
         __syncthreads();
     }
 }
 
-// cur: row cursors preset to the row offsets.
-__global__ void __launch_bounds__(PART_THREADS) part_rows(const uint2 *__restrict__ pairs, PartPlan plan, uint32_t n,
-                                                          unsigned long long *cur, uint32_t *col) {
-    extern __shared__ uint32_t rows_sm[];
+// With up to PART_STAGE_ROWS rows per bucket a tile is put in row order in shared
+// memory first (its columns, and the row of each), so that the entries of a row
+// leave together: 16 on average with 2,048 rows, 7 to 8 sectors a warp instead
+// of 32.  R-MAT 22 (134 M entries): 1.17 -> 0.60 ms; the direct form, one cursor
+// per row in shared memory, stays for more rows, where the counters leave no
+// room for a tile and its entries share few rows.
+constexpr uint32_t PART_STAGE_ROWS = 4096;
+constexpr size_t part_rows_smem(int shift) {
+    return (1u << shift) <= PART_STAGE_ROWS ? (size_t)PART_TILE * 6 + ((size_t)8 << shift) : (size_t)4 << shift;
+}
+template <bool STAGE>
+__global__ void __launch_bounds__(STAGE ? 1024 : PART_THREADS) part_rows(const uint2 *__restrict__ pairs, PartPlan plan,
+                                                                         uint32_t n, const int64_t *__restrict__ rowptr,
+                                                                         uint32_t *col) {
+    extern __shared__ __align__(16) unsigned char part_sm[];
+    constexpr uint32_t NT = STAGE ? 1024 : PART_THREADS;
     const uint32_t rows = 1u << plan.shift;
+    uint32_t *cur = reinterpret_cast<uint32_t *>(part_sm);  // next place of each row
+    // staged: distance from a place in the tile to the place in the bucket, per
+    // row; the tile's columns and rows in row order
+    uint32_t *delta = cur + rows, *stage = delta + rows;
+    uint16_t *row_of = reinterpret_cast<uint16_t *>(stage + PART_TILE);
+    __shared__ uint32_t wsum[NT / 32];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t tiles = plan.tile[plan.buckets];
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         uint64_t lo, hi;
         const uint32_t b = part_tile(plan, t, lo, hi);
-        const bool alone = plan.tile[b + 1] - plan.tile[b] == 1;
         const uint64_t base = plan.base[b];  // the bucket's rows hold entries [base, base of the next)
-        for (uint32_t i = threadIdx.x; i < rows; i += PART_THREADS) rows_sm[i] = 0;
-        __syncthreads();
+        const uint64_t r0 = (uint64_t)b << plan.shift, t0 = (uint64_t)t << plan.shift;
+        if constexpr (STAGE) {
+            constexpr uint32_t PER = PART_STAGE_ROWS / NT;
+            const uint32_t per = (rows + NT - 1) / NT, i0 = threadIdx.x * per;
+            uint32_t c[PER], own = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++) {
+                c[k] = k < per && i0 + k < rows && r0 + i0 + k < n ? plan.count[t0 + i0 + k] : 0u;
+                own += c[k];
+            }
+            uint32_t wtot;
+            uint32_t at = warp_excl_scan(own, lane, wtot);
+            if (lane == 0) wsum[warp] = wtot;
+            __syncthreads();
+            at += __reduce_add_sync(KC_FULL_MASK, lane < warp ? wsum[lane] : 0u);
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++)
+                if (c[k]) {
+                    cur[i0 + k] = at;
+                    delta[i0 + k] = (uint32_t)((uint64_t)rowptr[r0 + i0 + k] - base) + plan.off[t0 + i0 + k] - at;
+                    at += c[k];
+                }
+            __syncthreads();
 #pragma unroll 4
-        for (uint64_t e = lo + threadIdx.x; e < hi; e += PART_THREADS) atomicAdd(&rows_sm[pairs[e].x & (rows - 1)], 1u);
-        __syncthreads();
-        const uint64_t r0 = (uint64_t)b << plan.shift;
-        for (uint32_t i = threadIdx.x; i < rows && r0 + i < n; i += PART_THREADS) {
-            const uint32_t c = rows_sm[i];
-            if (c) rows_sm[i] = (uint32_t)((alone ? cur[r0 + i] : atomicAdd(&cur[r0 + i], (unsigned long long)c)) - base);
-        }
-        __syncthreads();
+            for (uint64_t e = lo + threadIdx.x; e < hi; e += NT) {
+                const uint2 q = pairs[e];
+                const uint32_t r = q.x & (rows - 1), p = atomicAdd(&cur[r], 1u);
+                stage[p] = q.y;
+                row_of[p] = (uint16_t)r;
+            }
+            __syncthreads();
+            const uint32_t len = (uint32_t)(hi - lo);
 #pragma unroll 4
-        for (uint64_t e = lo + threadIdx.x; e < hi; e += PART_THREADS) {
-            const uint2 q = pairs[e];
-            col[base + atomicAdd(&rows_sm[q.x & (rows - 1)], 1u)] = q.y;
+            for (uint32_t i = threadIdx.x; i < len; i += NT) col[base + (uint32_t)(delta[row_of[i]] + i)] = stage[i];
+        } else {
+            for (uint32_t i = threadIdx.x; i < rows && r0 + i < n; i += NT)
+                if (plan.count[t0 + i]) cur[i] = (uint32_t)((uint64_t)rowptr[r0 + i] - base) + plan.off[t0 + i];
+            __syncthreads();
+#pragma unroll 4
+            for (uint64_t e = lo + threadIdx.x; e < hi; e += NT) {
+                const uint2 q = pairs[e];
+                col[base + atomicAdd(&cur[q.x & (rows - 1)], 1u)] = q.y;
+            }
         }
         __syncthreads();
     }
@@ -449,7 +506,10 @@ static int part_smem_limits() {
     KC_CUDA(cudaFuncSetAttribute(part_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(2 * PART_EDGES * sizeof(uint2) + PART_MAX_BUCKETS * 12)));
     KC_CUDA(cudaFuncSetAttribute(part_degrees, cudaFuncAttributeMaxDynamicSharedMemorySize, rows));
-    KC_CUDA(cudaFuncSetAttribute(part_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, rows));
+    KC_CUDA(cudaFuncSetAttribute(part_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, rows));
+    int most = 0;
+    for (int shift = 0; 1u << shift <= PART_STAGE_ROWS; shift++) most = (int)part_rows_smem(shift);
+    KC_CUDA(cudaFuncSetAttribute(part_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     done[dev] = true;
     return KC_OK;
 }
@@ -1422,7 +1482,8 @@ int build_csr_from_edges(Graph *g, const uint32_t *d_src, const uint32_t *d_dst,
     cudaMemsetAsync(deg, 0, ((uint64_t)n + 1) * 4, s);
     cudaMemsetAsync(err, 0, 4, s);
     // partitioned where the order within a row is free and there is room for
-    // the pairs (16 bytes per edge)
+    // the pairs (16 bytes per edge) and the tiles' row shares (6 bytes per row of a
+    // bucket and tile: 0.8 bytes per edge with 2,048 rows, at most 6)
     PartPlan plan{};
     uint2 *pairs = nullptr;
     plan.shift = part_shift(m, n);
@@ -1430,10 +1491,15 @@ int build_csr_from_edges(Graph *g, const uint32_t *d_src, const uint32_t *d_dst,
         plan.buckets = ((n - 1) >> plan.shift) + 1;
         rc = dalloc(&plan.base, 3ull * (plan.buckets + 1), "partition plan");
         if (!rc) rc = dalloc(&pairs, 2 * m, "partitioned edges");
+        const uint64_t shares = (2 * m / PART_TILE + plan.buckets) << plan.shift;
+        if (!rc) rc = dalloc(&plan.off, shares, "row shares of the tiles");
+        if (!rc) rc = dalloc(&plan.count, shares, "row shares of the tiles");
         if (!rc) rc = part_smem_limits();
         if (rc) {
             dfree(plan.base);
             dfree(pairs);
+            dfree(plan.off);
+            dfree(plan.count);
             plan.shift = -1;
             pairs = nullptr;
             if (rc != KC_ERR_NOMEM) { dfree(deg); dfree(err); return rc; }
@@ -1445,6 +1511,8 @@ int build_csr_from_edges(Graph *g, const uint32_t *d_src, const uint32_t *d_dst,
         if (part) {
             dfree(plan.base);
             dfree(pairs);
+            dfree(plan.off);
+            dfree(plan.count);
         }
     };
     const int part_grid = sms * 2;
@@ -1465,7 +1533,7 @@ int build_csr_from_edges(Graph *g, const uint32_t *d_src, const uint32_t *d_dst,
     if (e != cudaSuccess) { dfree(deg); dfree(err); release_part(); return fail(KC_ERR_CUDA, "degree count: %s", cudaGetErrorString(e)); }
     if (herr) { dfree(deg); dfree(err); release_part(); return fail(KC_ERR_INVALID, "edge endpoint >= n (%u)", n); }
     if (part) {
-        part_pairs<<<(unsigned)std::min<uint64_t>((m + PART_EDGES - 1) / PART_EDGES, (uint64_t)part_grid), PART_THREADS,
+        part_pairs<<<(unsigned)std::min<uint64_t>((m + PART_EDGES - 1) / PART_EDGES, (uint64_t)sms), PAIR_THREADS,
                      2 * PART_EDGES * sizeof(uint2) + plan.buckets * 12, s>>>(d_src, d_dst, m, n, plan, pairs);
         part_degrees<<<row_grid, PART_THREADS, row_smem, s>>>(pairs, plan, n, deg);
     }
@@ -1477,12 +1545,15 @@ int build_csr_from_edges(Graph *g, const uint32_t *d_src, const uint32_t *d_dst,
     rc = dalloc(&g->col, g->nnz + 1, "column ids");
     if (rc) { dfree(deg); dfree(err); release_part(); return rc; }
     unsigned long long *cur = nullptr;  // row fill cursors, starting at the row offsets
-    if (m) {
+    if (part && (1u << plan.shift) <= PART_STAGE_ROWS) {
+        part_rows<true><<<sms, 1024, part_rows_smem(plan.shift), s>>>(pairs, plan, n, g->rowptr, g->col);
+    } else if (part) {
+        part_rows<false><<<row_grid, PART_THREADS, row_smem, s>>>(pairs, plan, n, g->rowptr, g->col);
+    } else if (m) {
         rc = dalloc(&cur, (uint64_t)n + 1, "row cursors");
         if (rc) { dfree(deg); dfree(err); release_part(); return rc; }
         cudaMemcpyAsync(cur, g->rowptr, ((uint64_t)n + 1) * 8, cudaMemcpyDeviceToDevice, s);
-        if (part) part_rows<<<row_grid, PART_THREADS, row_smem, s>>>(pairs, plan, n, cur, g->col);
-        else scatter_edges<<<grid_for(m, 256, sms), 256, 0, s>>>(d_src, d_dst, m, n, cur, g->col);
+        scatter_edges<<<grid_for(m, 256, sms), 256, 0, s>>>(d_src, d_dst, m, n, cur, g->col);
     }
     e = cudaStreamSynchronize(s);
     dfree(cur);
