@@ -108,28 +108,38 @@ __global__ void scan_sums_single(unsigned long long *sums, uint64_t count) {
 
 __global__ void scan_tile_apply(const uint32_t *__restrict__ in, int64_t *__restrict__ out, uint64_t n,
                                 const unsigned long long *sums) {
+    // a word of padding per 32 keeps the threads' runs of 8 off each other's
+    // banks, and the offsets leave through the same array, a warp's 32 at a time
+    constexpr int PAD = SCAN_TILE + SCAN_TILE / 32;
     __shared__ unsigned long long ws[33];
-    __shared__ uint32_t tile[SCAN_TILE];
+    __shared__ unsigned long long tile[PAD];
     uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-    for (int i = threadIdx.x; i < SCAN_TILE; i += SCAN_THREADS) {
-        uint64_t j = base + i;
-        tile[i] = j < n ? in[j] : 0u;
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; i++) {
+        const int k = i * SCAN_THREADS + threadIdx.x;
+        const uint64_t j = base + k;
+        tile[k + k / 32] = j < n ? in[j] : 0u;
     }
     __syncthreads();
+    const int k0 = threadIdx.x * SCAN_ITEMS + threadIdx.x * SCAN_ITEMS / 32;
     unsigned long long loc[SCAN_ITEMS];
     unsigned long long s = 0;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; i++) {
         loc[i] = s;
-        s += tile[threadIdx.x * SCAN_ITEMS + i];
+        s += tile[k0 + i];
     }
     unsigned long long tot;
     unsigned long long ex = block_excl_scan_u64(s, ws, tot);
     unsigned long long off = sums[blockIdx.x] + ex;
 #pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; i++) tile[k0 + i] = off + loc[i];
+    __syncthreads();
+#pragma unroll
     for (int i = 0; i < SCAN_ITEMS; i++) {
-        uint64_t j = base + (uint64_t)threadIdx.x * SCAN_ITEMS + i;
-        if (j < n) out[j] = (int64_t)(off + loc[i]);
+        const int k = i * SCAN_THREADS + threadIdx.x;
+        const uint64_t j = base + k;
+        if (j < n) out[j] = (int64_t)tile[k + k / 32];
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
         uint64_t tiles = gridDim.x;
@@ -1423,8 +1433,16 @@ __global__ void unique_rows(const int64_t *__restrict__ rowptr, uint32_t n, uint
 // ------------------------------------------------------- graph stats ------
 __global__ void degree_stats(const int64_t *__restrict__ rowptr, uint32_t n, uint32_t *maxdeg,
                              unsigned long long *vnodes) {
+    __shared__ uint32_t mx_sh;
+    __shared__ unsigned long long vn_sh;
+    if (threadIdx.x == 0) {
+        mx_sh = 0;
+        vn_sh = 0;
+    }
+    __syncthreads();
     uint32_t mx = 0;
     unsigned long long vn = 0;
+#pragma unroll 4
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t d = (uint64_t)(rowptr[v + 1] - rowptr[v]);
         mx = max(mx, (uint32_t)d);
@@ -1434,8 +1452,13 @@ __global__ void degree_stats(const int64_t *__restrict__ rowptr, uint32_t n, uin
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) vn += __shfl_xor_sync(KC_FULL_MASK, vn, o);
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(maxdeg, mx);
-        atomicAdd(vnodes, vn);
+        atomicMax(&mx_sh, mx);
+        atomicAdd(&vn_sh, vn);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMax(maxdeg, mx_sh);
+        atomicAdd(vnodes, vn_sh);
     }
 }
 
@@ -1445,7 +1468,8 @@ int graph_finish(Graph *g) {
     KC_TRY(dalloc(&md, 4, "graph stats"));
     unsigned long long *vn = reinterpret_cast<unsigned long long *>(md + 2);
     cudaMemsetAsync(md, 0, 16, s);
-    if (g->n) degree_stats<<<grid_for(g->n, 256, g->sm_count), 256, 0, s>>>(g->rowptr, g->n, md, vn);
+    // few CTAs: each ends with two atomics on the same two words
+    if (g->n) degree_stats<<<std::min(grid_for(g->n, 256, g->sm_count), std::max(g->sm_count, 1) * 4), 256, 0, s>>>(g->rowptr, g->n, md, vn);
     uint32_t h[4];
     cudaMemcpyAsync(h, md, 16, cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamSynchronize(s);
