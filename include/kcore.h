@@ -193,7 +193,7 @@ int kc_decompose(kc_graph *g, int method, uint32_t *core_out, int out_on_device,
 /* Chooses what KC_AUTO runs on this graph by timing it: the bucket peel
  * with its default tunables, the peel with the other row-chunk size (1024 /
  * 2048 entries), the peel keeping more cascade items per CTA ("peel.spill"
- * 2 x + 16), and the h-index iteration, each warmed up once and timed twice;
+ * 48, or 2 x + 16 where it was set), and the h-index iteration, each warmed up once and timed twice;
  * the fastest (method and peel tunables) is kept in the graph.  *method receives the chosen KC_*
  * method, *best_ms its time (either may be NULL).  The first
  * kc_decompose(KC_AUTO) of a graph calls this itself, so that call takes
@@ -208,7 +208,7 @@ int kc_graph_last_timing(const kc_graph *g, double *total_ms, double *kernel_ms)
  * the benchmarks use these).  Names: "peel.chunk" (row entries per peel work
  * item; 0, the default, picks 1024, or 2048 for graphs of 2^29 entries or
  * more), "peel.spill" (cascade items a CTA keeps before publishing to the
- * shared queues, default 16), "peel.steal" (most items reserved per steal,
+ * shared queues; until it is set, by the length of their rows), "peel.steal" (most items reserved per steal,
  * 1..64, default 32), "peel.queues" (number
  * of shared queues, 1..64), "peel.ctas_per_sm" (0 = occupancy maximum),
  * "peel.unroll" (row entries each lane keeps in flight, 4 or 8),

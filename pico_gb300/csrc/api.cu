@@ -510,7 +510,7 @@ static int autotune_graph(Graph *g, cudaStream_t s) {
     const int other_chunk = (g->nnz >= (1ull << 29)) ? 1024 : 2048;
     const Cand cands[] = {{KC_PEELONE_DYN, base.peel_chunk, base.peel_spill},
                           {KC_PEELONE_DYN, other_chunk, base.peel_spill},
-                          {KC_PEELONE_DYN, base.peel_chunk, 2 * base.peel_spill + 16},
+                          {KC_PEELONE_DYN, base.peel_chunk, base.peel_spill < 0 ? 48 : 2 * base.peel_spill + 16},
                           {KC_NBR, base.peel_chunk, base.peel_spill}};
     double best = 1e300;
     Cand pick = cands[0];

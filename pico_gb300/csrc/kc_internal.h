@@ -103,7 +103,7 @@ struct PeelTrace {
 
 struct Tuning {
     int peel_chunk = 0;  // 0: by graph size (1024 entries, 2048 from 2^29 entries up)
-    int peel_spill = 16;  // measured best with 32-item steals (R-MAT scale 22 and 25)
+    int peel_spill = -1;  // cascade items a CTA keeps; -1: by the length of their rows (peel.cu)
     int peel_steal = 32;
     int peel_queues = 1;
     int peel_ctas_per_sm = 0;

@@ -68,6 +68,17 @@ constexpr unsigned MIN_CHUNK = 256;   // smallest row chunk (sizes the shared qu
 // claimed vertices outweigh the round trip.  (Probes past the L1 throughout, as
 // before: 0.263, 1.256, 3.67, 5.63.)
 constexpr unsigned PROBE_MIN = 512;
+// How many items a CTA keeps before it publishes claims on the shared queues, by
+// the mean row length of the claims at hand: 16,384 entries' worth of rows of up
+// to 32 entries, 8,192 of rows up to 128, 4,096 of longer ones.  Publishing costs
+// two atomics on the same two words of all CTAs, which many short rows are not
+// worth; a few long rows are work enough for another CTA.  Kernel times (ms),
+// 16 items whatever their length -> this rule: uniform random 65,536 / 10^6 /
+// 4 x 10^6 vertices 0.247 / 1.21 / 4.28 -> 0.237 / 0.54 / 1.86, R-MAT 18 2.10 ->
+// 2.04, R-MAT 25 with a planted core 22.5 -> 22.1, R-MAT 22 5.60 -> 5.62.  With
+// 4,096 entries throughout 10^6 and 4 x 10^6 vertices take 0.77 and 2.39, with
+// 8,192 throughout R-MAT 22 and 25 take 5.73 and 22.7.
+constexpr unsigned SPILL_AUTO = ~0u, SPILL_ENTRIES = 16384, SPILL_MIN = 4, SPILL_MAX = 1024;
 constexpr unsigned long long SENT = ~0ull;
 constexpr unsigned int NO_LEVEL = 0xffffffffu;
 
@@ -97,7 +108,7 @@ struct PeelArgs {
     unsigned long long timeout_ns;
     uint32_t max_level_indices;
     unsigned chunk;              // row entries per work item
-    unsigned spill_t;            // cascade items a CTA keeps locally
+    unsigned spill_t;            // cascade items a CTA keeps locally, or SPILL_AUTO
     unsigned steal_max;          // items per steal
     unsigned nq;                 // shared queues in use
     unsigned round_e;            // balanced rounds: row entries a CTA takes per round
@@ -841,12 +852,19 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                             // overwrite this step's batch, which starts at b_base);
                             // otherwise publish them on a shared queue
                             const unsigned cnt = __popc(pb);
+                            unsigned keep = A.spill_t;
+                            if (keep == SPILL_AUTO) {
+                                const unsigned sum = __reduce_add_sync(
+                                    KC_FULL_MASK, push ? (unsigned)min(cr1[k] - cr0[k], (int64_t)RANGE_LEN) : 0u);
+                                const unsigned halves = (sum > 32 * cnt) + (sum > 128 * cnt);
+                                keep = min(SPILL_MAX, max(SPILL_MIN, (SPILL_ENTRIES >> halves) * cnt / max(sum, 1u)));
+                            }
                             unsigned slot_lo = 0, slot_hi = 0;
                             int spill = 0;
                             if (lane == 0) {
                                 unsigned t = q_tail;
                                 for (;;) {
-                                    if (t + cnt - b_base > QCAP || t + cnt - round_head > A.spill_t) { spill = 1; break; }
+                                    if (t + cnt - b_base > QCAP || t + cnt - round_head > keep) { spill = 1; break; }
                                     unsigned old = atomicCAS(&q_tail, t, t + cnt);
                                     if (old == t) break;
                                     t = old;
@@ -1025,7 +1043,7 @@ int peel_run(Graph *g, cudaStream_t s, bool gpp_zero_to_one_flag, kc_stats *st) 
     // measured: 1024-entry chunks on R-MAT scale 22 (128 M entries), 2048 on
     // R-MAT scale 25 (1.07 B entries, 4% faster than 1024)
     A.chunk = g->tune.peel_chunk ? (unsigned)g->tune.peel_chunk : (g->nnz >= (1ull << 29) ? 2048u : 1024u);
-    A.spill_t = (unsigned)g->tune.peel_spill;
+    A.spill_t = g->tune.peel_spill < 0 ? SPILL_AUTO : (unsigned)g->tune.peel_spill;
     A.steal_max = (unsigned)g->tune.peel_steal;
     A.nq = nq_of(g);
     A.round_e = (unsigned)g->tune.peel_round_entries;
