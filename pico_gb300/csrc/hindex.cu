@@ -56,8 +56,8 @@
 //     by all SMs at a time, and from the L1 they neither queue at their L2 slice
 //     nor take its latency: R-MAT 18 1.35 -> 1.24 ms, R-MAT 22 7.45 -> 6.32,
 //     R-MAT 25 with a planted core 67.2 -> 64.2; without hubs nothing is gained
-//     (Erdos-Renyi 10^6 / 8 x 10^6 1.18 -> 1.20).  The waits of the barrier are
-//     bounded.
+//     (Erdos-Renyi 10^6 / 8 x 10^6 1.18 -> 1.20).  The waits of the barrier
+//     (one per sweep, below) are bounded.
 #include <algorithm>
 
 #include "kc_device.cuh"
@@ -130,14 +130,14 @@ __global__ void hindex_init(const int64_t *__restrict__ rowptr, uint32_t n, uint
         unsigned b = __ballot_sync(KC_FULL_MASK, bigv);
         if (b) {
             unsigned long long p = 0;
-            if (lane == 0) p = atomicAdd(&ctl->big_len[0], (unsigned long long)__popc(b));
+            if (lane == 0) p = atomicAdd(&ctl->len[0].big, (unsigned long long)__popc(b));
             p = __shfl_sync(KC_FULL_MASK, p, 0);
             if (bigv) big0[p + __popc(b & lt)] = (uint32_t)v;
         }
         const unsigned bd = __ballot_sync(KC_FULL_MASK, medv);
         if (bd) {
             unsigned long long p = 0;
-            if (lane == 0) p = atomicAdd(&ctl->mid_len[0], (unsigned long long)__popc(bd));
+            if (lane == 0) p = atomicAdd(&ctl->len[0].mid, (unsigned long long)__popc(bd));
             p = __shfl_sync(KC_FULL_MASK, p, 0);
             if (medv) list0[n - (p + __popc(bd & lt))] = (uint32_t)v;
         }
@@ -297,6 +297,7 @@ __global__ void __launch_bounds__(HX_ORD_THREADS) hx_order_rows(const int64_t *_
 struct HxStage {
     uint32_t *buf;  // 64 entries
     unsigned cnt;   // the same on every lane, below 32 between calls
+    unsigned slot;  // of the next sweep's list lengths
 };
 
 __device__ __forceinline__ void hx_stage_push(const HxArgs &A, HxStage &st, bool take, uint32_t u, unsigned nxt,
@@ -308,7 +309,7 @@ __device__ __forceinline__ void hx_stage_push(const HxArgs &A, HxStage &st, bool
     if (st.cnt >= 32) {
         __syncwarp();
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&A.ctl->list_len[nxt], 32ull);
+        if (lane == 0) base = atomicAdd(&A.ctl->len[st.slot].list, 32ull);
         base = __shfl_sync(KC_FULL_MASK, base, 0);
         A.list[nxt][base + lane] = st.buf[lane];
         const uint32_t left = st.buf[32 + lane];
@@ -322,7 +323,7 @@ __device__ __forceinline__ void hx_stage_push(const HxArgs &A, HxStage &st, bool
 __device__ __forceinline__ void hx_stage_flush(const HxArgs &A, HxStage &st, unsigned nxt, unsigned lane) {
     if (st.cnt) {
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&A.ctl->list_len[nxt], (unsigned long long)st.cnt);
+        if (lane == 0) base = atomicAdd(&A.ctl->len[st.slot].list, (unsigned long long)st.cnt);
         base = __shfl_sync(KC_FULL_MASK, base, 0);
         if (lane < st.cnt) A.list[nxt][base + lane] = st.buf[lane];
         st.cnt = 0;
@@ -370,7 +371,7 @@ __device__ __forceinline__ void hx_activate_all(const HxArgs &A, const uint32_t 
             if (!m) continue;
             unsigned long long base = 0;
             if (lane == __ffs(m) - 1)
-                base = atomicAdd(q == 2 ? &A.ctl->big_len[nxt] : &A.ctl->mid_len[nxt], (unsigned long long)__popc(m));
+                base = atomicAdd(q == 2 ? &A.ctl->len[st.slot].big : &A.ctl->len[st.slot].mid, (unsigned long long)__popc(m));
             base = __shfl_sync(KC_FULL_MASK, base, __ffs(m) - 1);
             if (kind == q) {
                 const unsigned long long p = base + __popc(m & ((1u << lane) - 1u));
@@ -958,6 +959,42 @@ __device__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint3
 constexpr uint32_t HX_SMEM_WORDS =
     HX_WARPS * (HX_WARP_MAX + 1) > HX_BINS ? HX_WARPS * (HX_WARP_MAX + 1) : HX_BINS;
 
+// The end of sweep `gen`: arrivals are counted from the launch on, so nothing is
+// reset and the generation is known beforehand.  With one barrier per sweep
+// instead of two, and the lengths, cursors, arrivals, generation and error on
+// lines of their own (they shared two, and the waiting CTAs' polls met the others'
+// atomics there), the shortest sweep of R-MAT 22 takes 6.7 us instead of 12.2,
+// and the kernel on uniform random graphs of 65,536 / 10^6 vertices 0.36 / 1.00
+// instead of 0.51 / 1.25 ms, on R-MAT 18 / 22 0.89 / 6.05 instead of 1.26 / 6.30.
+__device__ __forceinline__ bool hx_barrier(HindexCtl *ctl, unsigned nblocks, unsigned gen, unsigned long long timeout_ns) {
+    __shared__ unsigned int ok_sh;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        fence_acq_rel();
+        unsigned int err = 0;
+        if (atomicAdd(&ctl->bar_count, 1u) == nblocks * (gen + 1u) - 1u) {
+            fence_acq_rel();
+            st_release(&ctl->bar_gen, gen + 1u);
+            err = ld_relaxed(&ctl->err);
+        } else {
+            const unsigned long long t0 = global_ns();
+            for (unsigned int spins = 0;;) {
+                err = ld_relaxed(&ctl->err);
+                if (ld_acquire(&ctl->bar_gen) == gen + 1u || err) break;
+                if ((++spins & 63u) == 0 && global_ns() - t0 > timeout_ns) {
+                    atomicCAS(&ctl->err, 0u, (unsigned)KC_ERR_TIMEOUT);
+                    err = KC_ERR_TIMEOUT;
+                    break;
+                }
+                __nanosleep(32);
+            }
+        }
+        ok_sh = err == 0;
+    }
+    __syncthreads();
+    return ok_sh != 0;
+}
+
 __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
     __shared__ uint32_t hist[HX_SMEM_WORDS];
     __shared__ uint32_t red[HX_WARPS];
@@ -968,7 +1005,7 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     HindexCtl *ctl = A.ctl;
     const unsigned G = gridDim.x;
-    HxStage st = {stage_sh[warp], 0u};
+    HxStage st = {stage_sh[warp], 0u, 0u};
     if (A.withhold && blockIdx.x == 0) {
         // The barrier count never reaches the grid size: the other CTAs' waits
         // run into their limit.  This CTA waits (bounded) for their verdict.
@@ -986,14 +1023,28 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
     }
     for (uint32_t sweep = 0;; sweep++) {
         const unsigned cur = sweep & 1, nxt = cur ^ 1;
-        if (threadIdx.x == 0) changed_sh = 0;
-        __syncthreads();
+        const unsigned slot = sweep % 3;
+        st.slot = slot == 2 ? 0u : slot + 1u;
         const bool tr = A.trace != nullptr && sweep < A.trace_cap;
         const unsigned long long t_sweep = tr ? global_ns() : 0ull;
         const bool all = sweep == 0 && A.first_all;
-        const unsigned long long nsmall = all ? (unsigned long long)A.n : ld_relaxed64(&ctl->list_len[cur]);
-        const unsigned long long nmid = ld_relaxed64(&ctl->mid_len[cur]);
-        const unsigned long long nbig = ld_relaxed64(&ctl->big_len[cur]);
+        const unsigned long long nsmall = all ? (unsigned long long)A.n : ld_relaxed64(&ctl->len[slot].list);
+        const unsigned long long nmid = ld_relaxed64(&ctl->len[slot].mid);
+        const unsigned long long nbig = ld_relaxed64(&ctl->len[slot].big);
+        // all CTAs read the same lengths: a sweep that queued nothing was the last
+        if (sweep && nsmall + nmid + nbig == 0) return;
+        if (sweep >= A.max_sweeps) {
+            if (threadIdx.x == 0) atomicCAS(&ctl->err, 0u, (unsigned)KC_ERR_CAPACITY);
+            return;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            // the slot of the sweep before is that of the sweep after the next
+            ctl->len[(sweep + 2) % 3] = HxLens{};
+            ctl->cur[(sweep + 2) % 3] = HxCursors{};
+            ctl->sweeps = sweep + 1;
+        }
+        if (threadIdx.x == 0) changed_sh = 0;
+        __syncthreads();
         if (tr && blockIdx.x == 0 && threadIdx.x == 0) {
             A.trace[sweep].t_start_ns = t_sweep;
             A.trace[sweep].level = sweep;
@@ -1002,7 +1053,7 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
         }
         // long rows: one CTA each, taken dynamically
         for (;;) {
-            if (threadIdx.x == 0) item_sh = atomicAdd(&ctl->big_cursor, 1ull);
+            if (threadIdx.x == 0) item_sh = atomicAdd(&ctl->cur[slot].big, 1ull);
             __syncthreads();
             unsigned long long i = item_sh;
             __syncthreads();
@@ -1029,7 +1080,7 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
         unsigned wchanged = 0;
         while (nmid) {
             unsigned long long i = 0;
-            if (lane == 0) i = atomicAdd(&ctl->mid_cursor, 1ull);
+            if (lane == 0) i = atomicAdd(&ctl->cur[slot].mid, 1ull);
             i = __shfl_sync(KC_FULL_MASK, i, 0);
             if (i >= nmid) break;
             const HxVertex x = hx_load(A, A.list[cur][A.n - i], cur, !all && lane == 0);
@@ -1037,7 +1088,7 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
         }
         for (;;) {
             unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(&ctl->cursor, (unsigned long long)grab);
+            if (lane == 0) base = atomicAdd(&ctl->cur[slot].list, (unsigned long long)grab);
             base = __shfl_sync(KC_FULL_MASK, base, 0);
             if (base >= nsmall) break;
             const unsigned cntv = (unsigned)(nsmall - base < grab ? nsmall - base : grab);
@@ -1075,7 +1126,6 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
         hx_stage_flush(A, st, nxt, lane);
         if (lane == 0 && wchanged) atomicAdd(&changed_sh, wchanged);
         __syncthreads();
-        if (threadIdx.x == 0 && changed_sh) atomicOr(&ctl->changed, 1u);
         const unsigned long long t_small = tr ? global_ns() : 0ull;
         if (tr && threadIdx.x == 0) {
             if (changed_sh) atomicAdd(&A.trace[sweep].claimed, changed_sh);
@@ -1083,31 +1133,8 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hindex_kernel(HxArgs A) {
             atomicAdd(&A.trace[sweep].cta_ns[1], t_small - t_big);
             atomicMax(&A.trace[sweep].t_work_end_ns, t_small);
         }
-        if (!grid_barrier(&ctl->bar_count, &ctl->bar_gen, G, &ctl->err, KC_ERR_TIMEOUT, A.timeout_ns)) return;
-        // one CTA resets the consumed lists; everyone reads the verdict after a second barrier
-        __shared__ unsigned int go_on;
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            ctl->list_len[cur] = 0;
-            ctl->mid_len[cur] = 0;
-            ctl->big_len[cur] = 0;
-            ctl->big_cursor = 0;
-            ctl->mid_cursor = 0;
-            ctl->cursor = 0;
-            ctl->sweeps = sweep + 1;
-            ctl->changed = 0;
-            // a sweep that lowered nothing queued nothing
-            unsigned long long pend = ctl->list_len[nxt] + ctl->mid_len[nxt] + ctl->big_len[nxt];
-            ctl->go_on = pend > 0 ? 1u : 0u;
-            if (sweep + 1 >= A.max_sweeps && pend > 0) atomicCAS(&ctl->err, 0u, (unsigned)KC_ERR_CAPACITY);
-            __threadfence();
-        }
-        if (!grid_barrier(&ctl->bar_count, &ctl->bar_gen, G, &ctl->err, KC_ERR_TIMEOUT, A.timeout_ns)) return;
-        // CTA 0 rewrites the flag only after the next sweep's first barrier,
-        // by which time every CTA has read it
-        if (threadIdx.x == 0) go_on = ld_relaxed(&ctl->go_on);
+        if (!hx_barrier(ctl, G, sweep, A.timeout_ns)) return;
         if (tr && threadIdx.x == 0) atomicAdd(&A.trace[sweep].cta_ns[2], global_ns() - t_small);
-        __syncthreads();
-        if (!go_on) return;
     }
 }
 
@@ -1291,8 +1318,8 @@ __global__ void hindex_seed(const int64_t *__restrict__ rowptr, const uint32_t *
         const uint32_t v = list[i];
         const unsigned bit = 1u << (v & 31);
         if (atomicOr(&inlist[v >> 5], bit) & bit) continue;  // listed twice
-        if (rowptr[v + 1] - rowptr[v] > (int64_t)HX_WARP_MAX) big0[atomicAdd(&ctl->big_len[0], 1ull)] = v;
-        else small0[atomicAdd(&ctl->list_len[0], 1ull)] = v;
+        if (rowptr[v + 1] - rowptr[v] > (int64_t)HX_WARP_MAX) big0[atomicAdd(&ctl->len[0].big, 1ull)] = v;
+        else small0[atomicAdd(&ctl->len[0].list, 1ull)] = v;
     }
 }
 

@@ -123,21 +123,23 @@ struct Tuning {
     int withhold = 0;  // failure-detection hook: one CTA never signals, so the others' waits run out
 };
 
-// Control block of the h-index iteration.
+// Control block of the h-index iteration.  Three sets of list lengths and
+// cursors take turns: a sweep reads one, fills the next and clears the third.
+struct alignas(128) HxLens {
+    unsigned long long list;  // active vertices of short rows
+    unsigned long long mid;   // of medium rows, stored from the far end of list[]
+    unsigned long long big;   // of long rows
+};
+struct alignas(128) HxCursors {
+    unsigned long long list, mid, big;
+};
 struct HindexCtl {
-    unsigned long long list_len[2];  // active list lengths (ping-pong)
-    unsigned long long big_len[2];   // high-degree active list lengths
-    unsigned long long mid_len[2];   // medium rows, stored from the far end of list[]
-    unsigned long long mid_cursor;   // work cursor (medium rows)
-    unsigned long long cursor;       // work cursor (short-row items)
-    unsigned long long big_cursor;   // work cursor (high-degree items)
-    unsigned int go_on;              // another sweep follows
-    unsigned int bar_count;          // grid barrier arrivals
-    unsigned int bar_gen;            // grid barrier generation
+    HxLens len[3];      // lists of sweep i: slot i % 3
+    HxCursors cur[3];
+    alignas(128) unsigned int bar_count;  // grid barrier arrivals since the launch
+    alignas(128) unsigned int bar_gen;    // grid barriers passed since the launch
+    alignas(128) unsigned int err;
     unsigned int sweeps;
-    unsigned int changed;
-    unsigned int err;
-    unsigned int err_info;
     unsigned long long ord_len;   // rows of 129..8192 entries given an ordered copy
     unsigned long long ord_huge;  // rows above 8192 entries given an ordered copy
     unsigned long long ord_cursor, ord_huge_cursor;  // work cursors of the copy
