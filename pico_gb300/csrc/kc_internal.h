@@ -77,13 +77,19 @@ struct alignas(128) PeelDone {
     unsigned long long word;
 };
 
+struct alignas(128) PeelCredits {
+    unsigned long long left;
+};
+
+// Words that are updated by all CTAs, words that idle CTAs poll and words that
+// are written now and then each have a line of their own.
 struct PeelCtl {
-    unsigned long long pending[3];   // outstanding work credits of level i
-    unsigned int next_min[3];        // smallest residual degree above level i
+    PeelCredits pending[3];          // outstanding work credits of level i
+    alignas(128) unsigned int next_min[3];  // smallest residual degree above level i
     unsigned int nonempty[3];        // some vertex was claimed at level i
-    unsigned int err;                // KC_ERR_* raised on the device
+    alignas(128) unsigned int err;   // KC_ERR_* raised on the device
     unsigned int err_info;           // where it was raised
-    unsigned int level_indices;      // level indices processed
+    alignas(128) unsigned int level_indices;  // level indices processed
     unsigned int levels;             // non-empty levels
     unsigned int kmax;               // largest level with a claim
     unsigned int zeros;              // degree-0 vertices (level 0)

@@ -153,7 +153,7 @@ __global__ void peel_ctl_reset(PeelCtl *ctl, unsigned int grid) {
     }
     if (t < 3) {
         ctl->done[t].word = 0;
-        ctl->pending[t] = grid;
+        ctl->pending[t].left = grid;
         ctl->next_min[t] = NO_LEVEL;
         ctl->nonempty[t] = 0;
     }
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
         if (tid == 0) {
             if (blockIdx.x == 0) {
                 unsigned s1 = (li + 1) % 3;
-                ctl->pending[s1] = G;
+                ctl->pending[s1].left = G;
                 ctl->next_min[s1] = NO_LEVEL;
                 ctl->nonempty[s1] = 0;
                 for (unsigned i = 0; i < A.nq; i++) {
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                             give -= 1;
                             withheld = 1;
                         }
-                        const unsigned long long had = atomicAdd(&ctl->pending[s], (unsigned long long)(0ull - give));
+                        const unsigned long long had = atomicAdd(&ctl->pending[s].left, (unsigned long long)(0ull - give));
                         credit = 0;
                         if (had == give && give) {
                             fence_acq_rel();
@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                         qi = __shfl_sync(KC_FULL_MASK, qi, 0);
                         unsigned long long pos = 0;
                         if (lane == 0) {
-                            atomicAdd(&ctl->pending[s], (unsigned long long)cnt);
+                            atomicAdd(&ctl->pending[s].left, (unsigned long long)cnt);
                             __threadfence();
                             pos = atomicAdd(&ctl->q[s][qi].tail, (unsigned long long)cnt);
                             if (pos + cnt > A.gq_cap) set_err(ctl, KC_ERR_CAPACITY, 3);
@@ -872,7 +872,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                                 unsigned long long p = t;
                                 if (spill) {
                                     const unsigned qi = atomicAdd(&spill_rr, 1u) % A.nq;
-                                    atomicAdd(&ctl->pending[s], (unsigned long long)cnt);
+                                    atomicAdd(&ctl->pending[s].left, (unsigned long long)cnt);
                                     __threadfence();
                                     p = atomicAdd(&ctl->q[s][qi].tail, (unsigned long long)cnt);
                                     if (p + cnt > A.gq_cap) { set_err(ctl, KC_ERR_CAPACITY, 4); spill = 2; }
