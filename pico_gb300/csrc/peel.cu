@@ -422,8 +422,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                     // word written once per level, on a line of its own: polls
                     // of the credit count would delay the credits still coming,
                     // and polls of the queues delay their producers, so those
-                    // are read one time in four (R-MAT 22: every 100 ns, all of
-                    // them, 5.88 ms; every 200 ns and one in four 5.60 ms).
+                    // are read every other time.  R-MAT 22 / R-MAT 25 with a
+                    // planted core: every 100 ns and every other time 5.26 /
+                    // 20.9 ms, every 200 ns 5.29 / 21.1, every 200 ns and one in
+                    // four 5.30 / 21.2.
                     if (A.trace) {
                         const unsigned long long now = global_ns();
                         mode_ns[prev_mode == M_SCAN ? 0 : prev_mode == M_PROC ? 1 : 2] += now - mode_t0;
@@ -433,7 +435,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                     for (unsigned polls = 0;;) {
                         const unsigned err = ld_relaxed(&ctl->err);
                         const unsigned long long done = ld_acquire64(&ctl->done[s].word);
-                        if (res_mask == 0 && (polls++ & 3u) == 0) {
+                        if (res_mask == 0 && (polls++ & 1u) == 0) {
                             for (unsigned k = 0; k < A.nq; k++) {
                                 const unsigned qi = (probe + k) % A.nq;
                                 unsigned long long h = ld_relaxed64(&ctl->q[s][qi].head);
@@ -483,7 +485,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                             md = M_EXIT;
                             break;
                         }
-                        __nanosleep(200);
+                        __nanosleep(100);
                     }
                 }
                 mode = md;
