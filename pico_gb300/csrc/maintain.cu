@@ -743,7 +743,8 @@ int graph_update(Graph *g, const uint32_t *ins_src, const uint32_t *ins_dst, uin
     const uint32_t n = g->n;
     // deletions alone need no matching rounds: the h-index iteration from the
     // old cores beats a full decomposition up to a few hundred thousand edges
-    // (R-MAT 22: 10^3 2.0 vs 8.4 ms, 10^5 6.3 vs 8.9 ms, 10^6 11.2 vs 10.6 ms)
+    // (R-MAT 22: 10^3 0.45 vs 5.6 ms, 10^4 0.99 vs 5.6, 10^5 5.3 vs 6.3, 5 x 10^5
+    // 8.1 vs 6.8; R-MAT 20: 5 x 10^5 3.7 vs 4.1, 10^6 4.5 vs 4.0)
     const bool incremental = n_ins + n_del <= (uint64_t)g->tune.update_incremental_max ||
                              (n_ins == 0 && n_del <= (uint64_t)g->tune.update_deletion_incremental_max);
     // The incremental path applies the deletions before it colours the
