@@ -797,7 +797,11 @@ __device__ int hx_block_suffix_find(const uint32_t *hist, int nb, uint64_t base,
 }
 
 // One CTA: recompute vertex v with a long row.
-__device__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint32_t *hist, uint32_t *red,
+// Not inlined: the long rows' code between the warps' loops costs these
+// registers and instruction fetches (kernel, inlined -> called: uniform random
+// 65,536 vertices 0.358 -> 0.338 ms, R-MAT 18 0.885 -> 0.866, R-MAT 22 6.03 ->
+// 5.97; hx_warp_vertex called: 6.58).
+__device__ __noinline__ bool hx_block_vertex(const HxArgs &A, uint32_t v, unsigned nxt, uint32_t *hist, uint32_t *red,
                                 HxStage &st) {
     const int64_t s = A.rowptr[v], e = A.rowptr[v + 1];
     __shared__ uint32_t cap_sh;
