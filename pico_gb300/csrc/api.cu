@@ -762,8 +762,8 @@ int kc_memcpy(void *dst, const void *src, size_t bytes, int kind) {
                                  : (kind == 2 ? cudaMemcpyDeviceToHost : (kind == 3 ? cudaMemcpyDeviceToDevice : cudaMemcpyDefault));
     if (kind < 1 || kind > 3) return fail(KC_ERR_INVALID, "copy kind %d", kind);
     KC_CUDA(cudaMemcpy(dst, src, bytes, k));
-    // a device-to-device cudaMemcpy may return before the copy is done
-    if (kind == 3) KC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    // a cudaMemcpy to the device may return before the copy is done
+    if (kind != 2) KC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return KC_OK;
 }
 

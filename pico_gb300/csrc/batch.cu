@@ -628,7 +628,6 @@ static int plan(kc_batch *b) {
         if (rc) return rc;
         c.grid = (int)std::min<size_t>((size_t)grid, c.order.size());
         KC_TRY(dalloc(&c.d_order, c.order.size(), "batch class order"));
-        KC_CUDA(cudaMemcpy(c.d_order, c.order.data(), c.order.size() * 4, cudaMemcpyHostToDevice));
         if (c.kind == BATCH_GLOBAL && !b->d_gdeg) {
             // every graph's part starts at a multiple of 8 vertices
             KC_TRY(dalloc(&b->d_gdeg, (uint64_t)b->g->n + 8ull * b->G + 8, "batch global degrees"));
@@ -636,6 +635,12 @@ static int plan(kc_batch *b) {
         }
         b->classes.push_back(std::move(c));
     }
+    for (BatchClass &c : b->classes)
+        KC_CUDA(cudaMemcpyAsync(c.d_order, c.order.data(), c.order.size() * 4, cudaMemcpyHostToDevice, b->g->stream));
+    // The launches may be on any stream, and a plain cudaMemcpy of a few bytes
+    // returns before they are on the device: behind other threads' uploads they
+    // arrive after a kernel on a non-blocking stream has started.
+    KC_CUDA(cudaStreamSynchronize(b->g->stream));
     b->planned = true;
     return KC_OK;
 }

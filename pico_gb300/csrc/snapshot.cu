@@ -238,6 +238,7 @@ int kc_graph_load(const char *path, int device, kc_graph **out) {
         int rc = dalloc(&g->core, h.n + 1, "core");
         if (!rc) {
             cudaError_t e = cudaMemcpy(g->core, base + b_row + b_col + pad, b_core, cudaMemcpyHostToDevice);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // the graph's stream does not wait for it
             if (e != cudaSuccess) rc = fail(KC_ERR_CUDA, "core upload: %s", cudaGetErrorString(e));
         }
         if (rc) {
