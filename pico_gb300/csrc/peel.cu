@@ -78,7 +78,19 @@ constexpr unsigned PROBE_MIN = 512;
 // 2.04, R-MAT 25 with a planted core 22.5 -> 22.1, R-MAT 22 5.60 -> 5.62.  With
 // 4,096 entries throughout 10^6 and 4 x 10^6 vertices take 0.77 and 2.39, with
 // 8,192 throughout R-MAT 22 and 25 take 5.73 and 22.7.
-constexpr unsigned SPILL_AUTO = ~0u, SPILL_ENTRIES = 16384, SPILL_MIN = 4, SPILL_MAX = 1024;
+// While an idle CTA has no published item to take, at most SPILL_IDLE items are
+// kept: a cascade that starts in few places (the corners of a grid, the first hub
+// of a core) otherwise stays on the CTAs that it happens to reach.  Kernel times
+// (ms) with 16 items whatever their length / the rule by row entries alone / with
+// this limit: grids of 1,000 and 2,000 squared 5.25 and 12.7 / 8.2 and 28.3 / 4.9
+// and 11.5-12.4, with diagonals 1,500 squared 11.5 / 57 / 10.2, a cube of 100
+// 1.74 / 3.66 / 1.15, Barabasi-Albert 10^6 x 8 and 500,000 x 16 1.56 and 1.27 /
+// 2.13 and 2.48 / 1.21 and 1.29; what has work everywhere is the same or pays for
+// the look at the count: uniform random 65,536 0.227 -> 0.223, R-MAT 22 5.25 ->
+// 5.30, R-MAT 25 with a planted core 20.8 -> 21.0.  A limit of 8 items doubles the
+// grids' times; a lower line than every CTA is slower on the grids and the cubes,
+// twice as high a line on the uniform random graphs (10^6 x 3 0.17 -> 0.50).
+constexpr unsigned SPILL_AUTO = ~0u, SPILL_ENTRIES = 16384, SPILL_MIN = 4, SPILL_MAX = 1024, SPILL_IDLE = 16;
 constexpr unsigned long long SENT = ~0ull;
 constexpr unsigned int NO_LEVEL = 0xffffffffu;
 
@@ -209,6 +221,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
     __shared__ unsigned long long wait_t0;
     __shared__ unsigned int withheld;
     __shared__ unsigned int rounds_sh;
+    __shared__ unsigned int idle_sh;  // when the last round began, an idle CTA had nothing to take
     __shared__ unsigned long long mode_ns[4], mode_t0;  // trace: time per mode in this level
     __shared__ int prev_mode;
     __shared__ unsigned int bal_off[BAL ? NT + 1 : 1];  // balanced rounds: item offsets,
@@ -284,6 +297,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
             claimed_any = 0;
             wait_t0 = 0;
             rounds_sh = 0;
+            idle_sh = 0;
             if (A.trace) {
                 mode_ns[0] = mode_ns[1] = mode_ns[2] = mode_ns[3] = 0;
                 mode_t0 = global_ns();
@@ -519,7 +533,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                 __syncthreads();
                 if (tid == 0) {
                     q_tail = qt + steal_cnt;
-                    credit += steal_cnt;
+                    // all credits but one go back: the level's count is then
+                    // the CTAs at work plus the items nobody has taken yet
+                    const unsigned long long spare = credit + steal_cnt - 1;
+                    credit = 1;
+                    if (spare) atomicAdd(&ctl->pending[s].left, 0ull - spare);
                     steal_cnt = 0;
                 }
                 __syncthreads();
@@ -633,6 +651,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
             // never outlasts a few dependent memory round trips and a claim
             // made in it is picked up in the next round.
             {
+                // read now, used by the next round, so that nobody waits for it (the low word is all of it)
+                const unsigned at_work =
+                    tid == NT - 32 ? ld_relaxed(reinterpret_cast<unsigned *>(&ctl->pending[s].left)) : 0u;
                 // the CTA queue's head once this round's items are taken (the
                 // spill threshold counts the items queued behind it)
                 unsigned round_head = q_head;
@@ -860,6 +881,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                                     KC_FULL_MASK, push ? (unsigned)min(cr1[k] - cr0[k], (int64_t)RANGE_LEN) : 0u);
                                 const unsigned halves = (sum > 32 * cnt) + (sum > 128 * cnt);
                                 keep = min(SPILL_MAX, max(SPILL_MIN, (SPILL_ENTRIES >> halves) * cnt / max(sum, 1u)));
+                                if (idle_sh) keep = min(keep, SPILL_IDLE);
                             }
                             unsigned slot_lo = 0, slot_hi = 0;
                             int spill = 0;
@@ -903,6 +925,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                 local_min = __reduce_min_sync(KC_FULL_MASK, local_min);
                 if (lane == 0 && local_min != NO_LEVEL) atomicMin(&min_sh, local_min);
                 if (lane == 0 && nit) claimed_any = 1;
+                if (tid == NT - 32) idle_sh = at_work < G;
                 if (A.trace && lane == 0 && wclaims) atomicAdd(&claims_sh, wclaims);
             }
             __syncthreads();
