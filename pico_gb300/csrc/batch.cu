@@ -555,7 +555,8 @@ static int batch_smem_limit() {
 template <typename DegT, bool SMEM>
 static int class_grid(int threads, size_t smem, int sms, int *grid) {
     auto fn = batch_peel<DegT, SMEM>;
-    if (smem > 48 * 1024) KC_TRY((batch_smem_limit<DegT, SMEM>()));
+    // whatever the size: 48 KB without the opt-in count the static variables too
+    KC_TRY((batch_smem_limit<DegT, SMEM>()));
     int occ = 0;
     KC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem));
     if (occ < 1) return fail(KC_ERR_UNSUPPORTED, "batch kernel (%d threads, %zu B shared) cannot be resident", threads, smem);
