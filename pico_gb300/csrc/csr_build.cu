@@ -795,7 +795,8 @@ static int build_in_order(Graph *g, const uint32_t *d_src, const uint32_t *d_dst
     if (rc) return done(rc);
     cudaMemsetAsync(state, 0, 16, s);
     cudaMemsetAsync(deg, 0, ((uint64_t)n + 1) * 4, s);
-    for (int p = 0; p < passes; p++) {
+    // a list of self-loops alone leaves nothing to sort, and no tile to divide by
+    for (int p = 0; p < passes && (p == 0 || g->nnz); p++) {
         OrderPass P{};
         P.src = d_src;
         P.dst = d_dst;
@@ -830,7 +831,7 @@ static int build_in_order(Graph *g, const uint32_t *d_src, const uint32_t *d_dst
             if (rc) return done(rc);
             if (last) order_place<true, true><<<ctas, ORDER_THREADS, sm, s>>>(P, nullptr, g->col, rows);
             else order_place<true, false><<<ctas, ORDER_THREADS, sm, s>>>(P, buf[0], nullptr, nullptr);
-        } else if (g->nnz) {
+        } else {
             order_hist<false><<<ctas, ORDER_THREADS, hist_sm, s>>>(P, nullptr);
             order_scan<<<scan_ctas, 1024, 0, s>>>(P, ctas, nullptr);
             if (last) order_place<false, true><<<ctas, ORDER_THREADS, sm, s>>>(P, nullptr, g->col, rows);
