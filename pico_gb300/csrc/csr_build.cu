@@ -553,20 +553,22 @@ struct OrderPass {
     uint64_t count;             // places of the sequence (first pass: 2 per line)
     uint64_t stretch;           // places per CTA, whole tiles
     uint32_t n;
+    uint32_t row0, rows;        // first pass: entries of rows [row0, row0 + rows); pairs count rows from row0
     int shift, bits;
     uint32_t *hist;             // [CTAs][2^bits]
     uint32_t *total;            // [2^bits]
 };
 
-// Place e of the sequence; false where it holds no entry (a self-loop, a bad id).
+// Place e of the sequence; false where it holds no entry of these rows (a
+// self-loop, a bad id, another row).
 template <bool EDGES>
 __device__ __forceinline__ bool order_entry(const OrderPass &P, uint64_t e, uint32_t &row, uint32_t &col) {
     if (e >= P.count) return false;
     if (EDGES) {
         const uint32_t a = P.src[e >> 1], b = P.dst[e >> 1];
-        row = e & 1 ? b : a;
+        row = (e & 1 ? b : a) - P.row0;
         col = e & 1 ? a : b;
-        return a != b && a < P.n && b < P.n;
+        return a != b && row < P.rows && col < P.n;  // the rows are below n
     }
     const uint2 q = P.in[e];
     row = q.x;
@@ -585,7 +587,7 @@ __global__ void __launch_bounds__(ORDER_THREADS) order_hist(OrderPass P, unsigne
     for (uint64_t e = lo + threadIdx.x; e < hi; e += ORDER_THREADS) {
         uint32_t row = 0, col = 0;
         if (order_entry<EDGES>(P, e, row, col)) atomicAdd(&order_sm[(row >> P.shift) & (bins - 1)], 1u);
-        else if (EDGES && (row >= P.n || col >= P.n)) atomicCAS(err, 0u, 1u);
+        else if (EDGES && err && (row >= P.n || col >= P.n)) atomicCAS(err, 0u, 1u);  // row0 is 0 where err is set
     }
     __syncthreads();
     for (uint32_t d = threadIdx.x; d < bins; d += ORDER_THREADS) P.hist[(uint64_t)blockIdx.x * bins + d] = order_sm[d];
@@ -767,82 +769,128 @@ static int order_smem_limits() {
     return KC_OK;
 }
 
-// Builds g's rows in edge-list order (m > 0).  Device arrays freed on return.
-static int build_in_order(Graph *g, const uint32_t *d_src, const uint32_t *d_dst, uint64_t m, uint32_t n) {
-    cudaStream_t s = g->stream;
-    const uint64_t stretches = (uint64_t)g->sm_count;  // CTAs of a pass, at most: one per SM
-    int bits = 1;
-    while (bits < 32 && ((uint64_t)n - 1) >> bits) bits++;
-    const int passes = (bits + ORDER_MAX_BITS - 1) / ORDER_MAX_BITS;
-    const int digit = (bits + passes - 1) / passes;
+struct OrderBuild {
+    Graph *g;
+    const uint32_t *src, *dst;
+    uint64_t m;
+    uint64_t stretches;         // CTAs of a pass, at most: one per SM
     uint32_t *hist = nullptr, *deg = nullptr, *rows = nullptr;
     unsigned long long *state = nullptr;  // entries, error flag
     uint2 *buf[2] = {nullptr, nullptr};
-    auto done = [&](int rc) {
-        cudaStreamSynchronize(s);
-        dfree(hist);
-        dfree(deg);
+    uint64_t done = 0;          // entries placed
+
+    // the sort that used them has ended
+    void free_sort() {
         dfree(rows);
-        dfree(state);
         dfree(buf[0]);
         dfree(buf[1]);
-        return rc;
-    };
-    int rc = order_smem_limits();
-    if (!rc) rc = dalloc(&hist, (stretches + 1) << digit, "digit counts");
-    if (!rc) rc = dalloc(&state, 2, "entry count");
-    if (!rc) rc = dalloc(&deg, (uint64_t)n + 1, "degrees");
-    if (rc) return done(rc);
-    cudaMemsetAsync(state, 0, 16, s);
-    cudaMemsetAsync(deg, 0, ((uint64_t)n + 1) * 4, s);
+        rows = nullptr;
+        buf[0] = buf[1] = nullptr;
+    }
+    ~OrderBuild() {
+        cudaStreamSynchronize(g->stream);
+        free_sort();
+        dfree(hist);
+        dfree(deg);
+        dfree(state);
+    }
+};
+
+// Sorts the entries of rows [row0, row0 + rows) behind those already placed.
+// All rows at once (row0 = 0, rows = n) also checks the ids and allocates the
+// columns.  The sort takes 4 bytes per entry for the rows, 8 for the pairs (from
+// 2^11 rows up) and 8 more above 2^22 rows, beside the 4 of the columns; where
+// they are not free, the two halves of the rows follow one after the other, each
+// reading the whole edge list.
+static int order_range(OrderBuild &B, uint32_t row0, uint32_t rows) {
+    Graph *g = B.g;
+    cudaStream_t s = g->stream;
+    const bool all = row0 == 0 && rows == g->n;
+    int bits = 1;
+    while (bits < 32 && ((uint64_t)rows - 1) >> bits) bits++;
+    const int passes = (bits + ORDER_MAX_BITS - 1) / ORDER_MAX_BITS;
+    const int digit = (bits + passes - 1) / passes;
+    unsigned long long h[2] = {0, 0};
     // a list of self-loops alone leaves nothing to sort, and no tile to divide by
-    for (int p = 0; p < passes && (p == 0 || g->nnz); p++) {
+    for (int p = 0; p < passes && (p == 0 || h[0]); p++) {
         OrderPass P{};
-        P.src = d_src;
-        P.dst = d_dst;
-        P.in = buf[(p + 1) & 1];
-        P.count = p ? g->nnz : 2 * m;
-        P.n = n;
+        P.src = B.src;
+        P.dst = B.dst;
+        P.in = B.buf[(p + 1) & 1];
+        P.count = p ? h[0] : 2 * B.m;
+        P.n = g->n;
+        P.row0 = row0;
+        P.rows = rows;
         P.shift = p * digit;
         P.bits = std::min(digit, bits - P.shift);
         const uint64_t tiles = (P.count + ORDER_TILE - 1) / ORDER_TILE;
-        const uint64_t per = (tiles + stretches - 1) / stretches;
+        const uint64_t per = (tiles + B.stretches - 1) / B.stretches;
         P.stretch = per * ORDER_TILE;
         const uint32_t ctas = (uint32_t)((tiles + per - 1) / per);
-        P.hist = hist;
-        P.total = hist + (stretches << digit);
+        P.hist = B.hist;
+        P.total = B.hist + (B.stretches << ORDER_MAX_BITS);
         const size_t sm = order_smem(P.bits);
         const size_t hist_sm = (size_t)4 << P.bits;
         const uint32_t scan_ctas = ((1u << P.bits) + 31) / 32;
         const bool last = p + 1 == passes;
+        uint32_t *col = g->col ? g->col + B.done : nullptr;
         if (p == 0) {
-            order_hist<true><<<ctas, ORDER_THREADS, hist_sm, s>>>(P, reinterpret_cast<unsigned int *>(state + 1));
-            order_scan<<<scan_ctas, 1024, 0, s>>>(P, ctas, state);
-            unsigned long long h[2] = {0, 0};
-            cudaMemcpyAsync(h, state, 16, cudaMemcpyDeviceToHost, s);
+            cudaMemsetAsync(B.state, 0, 16, s);
+            order_hist<true><<<ctas, ORDER_THREADS, hist_sm, s>>>(P, all ? reinterpret_cast<unsigned int *>(B.state + 1) : nullptr);
+            order_scan<<<scan_ctas, 1024, 0, s>>>(P, ctas, B.state);
+            cudaMemcpyAsync(h, B.state, 16, cudaMemcpyDeviceToHost, s);
             cudaError_t e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) return done(fail(KC_ERR_CUDA, "degree count: %s", cudaGetErrorString(e)));
-            if (h[1]) return done(fail(KC_ERR_INVALID, "edge endpoint >= n (%u)", n));
-            g->nnz = h[0];
-            rc = dalloc(&g->col, g->nnz + 1, "column ids");
-            if (!rc) rc = dalloc(&rows, g->nnz + 1, "row ids");
-            if (!rc && passes > 1) rc = dalloc(&buf[0], g->nnz + 1, "ordered pairs");
-            if (!rc && passes > 2) rc = dalloc(&buf[1], g->nnz + 1, "ordered pairs");
-            if (rc) return done(rc);
-            if (last) order_place<true, true><<<ctas, ORDER_THREADS, sm, s>>>(P, nullptr, g->col, rows);
-            else order_place<true, false><<<ctas, ORDER_THREADS, sm, s>>>(P, buf[0], nullptr, nullptr);
+            if (e != cudaSuccess) return fail(KC_ERR_CUDA, "degree count: %s", cudaGetErrorString(e));
+            if (h[1]) return fail(KC_ERR_INVALID, "edge endpoint >= n (%u)", g->n);
+            if (all) {
+                g->nnz = h[0];
+                KC_TRY(dalloc(&g->col, g->nnz + 1, "column ids"));
+                col = g->col;
+            }
+            B.free_sort();  // of the rows before, which the wait above covers
+            int rc = dalloc(&B.rows, h[0] + 1, "row ids");
+            if (!rc && passes > 1) rc = dalloc(&B.buf[0], h[0] + 1, "ordered pairs");
+            if (!rc && passes > 2) rc = dalloc(&B.buf[1], h[0] + 1, "ordered pairs");
+            if (rc == KC_ERR_NOMEM && rows > 1) {
+                clear_error();
+                B.free_sort();
+                KC_TRY(order_range(B, row0, rows / 2));
+                return order_range(B, row0 + rows / 2, rows - rows / 2);
+            }
+            if (rc) return rc;
+            if (last) order_place<true, true><<<ctas, ORDER_THREADS, sm, s>>>(P, nullptr, col, B.rows);
+            else order_place<true, false><<<ctas, ORDER_THREADS, sm, s>>>(P, B.buf[0], nullptr, nullptr);
         } else {
             order_hist<false><<<ctas, ORDER_THREADS, hist_sm, s>>>(P, nullptr);
             order_scan<<<scan_ctas, 1024, 0, s>>>(P, ctas, nullptr);
-            if (last) order_place<false, true><<<ctas, ORDER_THREADS, sm, s>>>(P, nullptr, g->col, rows);
-            else order_place<false, false><<<ctas, ORDER_THREADS, sm, s>>>(P, buf[p & 1], nullptr, nullptr);
+            if (last) order_place<false, true><<<ctas, ORDER_THREADS, sm, s>>>(P, nullptr, col, B.rows);
+            else order_place<false, false><<<ctas, ORDER_THREADS, sm, s>>>(P, B.buf[p & 1], nullptr, nullptr);
         }
     }
-    if (g->nnz) order_degrees<<<grid_for(g->nnz, 256, g->sm_count), 256, 0, s>>>(rows, g->nnz, deg);
-    rc = exclusive_scan_u32_i64(deg, g->rowptr, n, s);
+    if (h[0]) order_degrees<<<grid_for(h[0], 256, g->sm_count), 256, 0, s>>>(B.rows, h[0], B.deg + row0);
+    B.done += h[0];
+    return KC_OK;
+}
+
+// Builds g's rows in edge-list order (m > 0).
+static int build_in_order(Graph *g, const uint32_t *d_src, const uint32_t *d_dst, uint64_t m, uint32_t n) {
+    cudaStream_t s = g->stream;
+    OrderBuild B;
+    B.g = g;
+    B.src = d_src;
+    B.dst = d_dst;
+    B.m = m;
+    B.stretches = (uint64_t)g->sm_count;
+    KC_TRY(order_smem_limits());
+    KC_TRY(dalloc(&B.hist, (B.stretches + 1) << ORDER_MAX_BITS, "digit counts"));
+    KC_TRY(dalloc(&B.state, 2, "entry count"));
+    KC_TRY(dalloc(&B.deg, (uint64_t)n + 1, "degrees"));
+    cudaMemsetAsync(B.deg, 0, ((uint64_t)n + 1) * 4, s);
+    KC_TRY(order_range(B, 0, n));
+    KC_TRY(exclusive_scan_u32_i64(B.deg, g->rowptr, n, s));
     const cudaError_t e = cudaGetLastError();
-    if (!rc && e != cudaSuccess) rc = fail(KC_ERR_CUDA, "ordered rows: %s", cudaGetErrorString(e));
-    return done(rc);
+    if (e != cudaSuccess) return fail(KC_ERR_CUDA, "ordered rows: %s", cudaGetErrorString(e));
+    return KC_OK;
 }
 
 // ------------------------------------------------------ segmented sort ----

@@ -1,0 +1,58 @@
+"""Builds where device memory runs short: what the fast path takes beside the
+graph is not free, and the build without it gives the same rows.  The memory is
+taken by a buffer, in a process of its own, down to a stated rest."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+RUN = """
+import sys
+sys.path[:0] = [%r, %r]
+import numpy as np
+import torch
+import pico_gb300 as pg
+from test_gpu_build_rows import expected
+n, m, how, rest = int(sys.argv[1]), int(sys.argv[2]), sys.argv[3], int(sys.argv[4])
+rng = np.random.default_rng(m)
+
+
+def edges(m):
+    s, d = rng.integers(0, n, (2, m)).astype(np.uint32)
+    s[::5] = s[0]  # a long row
+    return s, d
+
+
+def build(s, d):
+    return pg.Graph.from_edges_device(s.data_ptr(), d.data_ptr(), s.numel(), n, dedup=how == "dedup", sort_rows=how == "sort")
+
+
+few, (s, d) = edges(1 << 20), edges(m)
+few, dev = ([torch.from_numpy(x.view(np.int32)).cuda() for x in e] for e in (few, (s, d)))
+torch.cuda.synchronize()
+build(*few).free()  # the kernels are loaded
+torch.cuda.empty_cache()
+held = torch.empty(torch.cuda.mem_get_info()[0] - (rest << 20), dtype=torch.uint8, device="cuda")
+rowptr, col = build(*dev).csr()
+keep = s != d
+want = expected(n, s[keep], d[keep], how)
+assert np.array_equal(rowptr, want[0]) and np.array_equal(col, want[1])
+print("exact")
+""" % (ROOT, os.path.join(ROOT, "tests"))
+
+
+def run(n, m, how, rest):
+    pytest.importorskip("torch")
+    r = subprocess.run([sys.executable, "-c", RUN, str(n), str(m), how, str(rest)], capture_output=True, text=True)
+    assert r.returncode == 0 and "exact" in r.stdout, r.stderr[-2000:]
+
+
+# 2^24 lines: 134 MB of columns; rows and pairs of the sort take 403 MB more for
+# all rows at once (537 above 2^22 vertices)
+@pytest.mark.parametrize("n, rest", [(1 << 20, 330), (5000000, 400)])
+def test_edge_list_order_by_row_ranges(n, rest):
+    run(n, 1 << 24, "keep", rest)
