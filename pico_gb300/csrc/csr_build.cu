@@ -1579,7 +1579,7 @@ int build_csr_from_edges(Graph *g, const uint32_t *d_src, const uint32_t *d_dst,
             clear_error();
         }
     }
-    const bool part = plan.shift >= 0;
+    bool part = plan.shift >= 0;
     auto release_part = [&]() {
         if (part) {
             dfree(plan.base);
@@ -1616,6 +1616,14 @@ int build_csr_from_edges(Graph *g, const uint32_t *d_src, const uint32_t *d_dst,
     cudaMemcpy(&nnz, g->rowptr + n, 8, cudaMemcpyDeviceToHost);
     g->nnz = (uint64_t)nnz;
     rc = dalloc(&g->col, g->nnz + 1, "column ids");
+    if (rc == KC_ERR_NOMEM && part) {
+        // the partition holds twice the columns: without it they may fit, and
+        // the edges are scattered by the row offsets that it gave
+        release_part();
+        part = false;
+        clear_error();
+        rc = dalloc(&g->col, g->nnz + 1, "column ids");
+    }
     if (rc) { dfree(deg); dfree(err); release_part(); return rc; }
     unsigned long long *cur = nullptr;  // row fill cursors, starting at the row offsets
     if (part && (1u << plan.shift) <= PART_STAGE_ROWS) {

@@ -56,3 +56,10 @@ def run(n, m, how, rest):
 @pytest.mark.parametrize("n, rest", [(1 << 20, 330), (5000000, 400)])
 def test_edge_list_order_by_row_ranges(n, rest):
     run(n, 1 << 24, "keep", rest)
+
+
+# the partition takes 290 MB, the columns 134 MB more, scattering and sorting
+# without it 305 MB in all
+@pytest.mark.parametrize("how", ["sort", "dedup"])
+def test_columns_that_fit_without_the_partition(how):
+    run(1 << 20, 1 << 24, how, 345)
