@@ -344,8 +344,8 @@ int kc_graph_from_segment(const kc_graph *g, uint32_t lo, uint32_t hi, kc_graph 
  * max_batch_graphs / max_batch_bytes) into one batched launch.  Inputs are
  * copied at submission: graphs of 256 KB and more to the device, as long as
  * all admitted requests fit in decompose_slots * max_batch_bytes and in the
- * free memory, else to host memory.  Latency = submission to result on the
- * host. */
+ * free memory, else to host memory.  Latency = submission (the start of the
+ * submitting call, so with that copy) to result on the host. */
 typedef struct kc_server kc_server;
 typedef struct kc_server_config {
     uint32_t decompose_slots;   /* concurrent decomposition lanes (default 2) */

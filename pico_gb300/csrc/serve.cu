@@ -476,11 +476,8 @@ static uint64_t submit(kc_server *S, Request *r) {
     std::lock_guard<std::mutex> lk(S->mu);
     if (r->kind == 1 && !r->admitted && r->large()) S->held_large++;
     r->ticket = S->next_ticket++;
-    r->t_submit = Clock::now();
-    if (!S->started) {
-        S->started = true;
-        S->t_first = r->t_submit;
-    }
+    if (!S->started || r->t_submit < S->t_first) S->t_first = r->t_submit;
+    S->started = true;
     S->reqs[r->ticket] = r;
     (r->kind == 0 ? S->upd_q : S->dec_q).push_back(r);
     S->cv_work.notify_all();
@@ -538,6 +535,7 @@ int kc_server_submit_update(kc_server *S, const uint32_t *ins_src, const uint32_
         return fail(KC_ERR_INVALID, "null argument");
     Request *r = new (std::nothrow) Request();
     if (!r) return fail(KC_ERR_NOMEM, "request");
+    r->t_submit = Clock::now();
     r->kind = 0;
     r->is.assign(ins_src, ins_src + n_ins);
     r->id.assign(ins_dst, ins_dst + n_ins);
@@ -556,6 +554,7 @@ int kc_server_submit_decompose(kc_server *S, const int64_t *rowptr, const uint32
     if (nnz < 0 || (nnz && !col)) return fail(KC_ERR_INVALID, "bad CSR");
     Request *r = new (std::nothrow) Request();
     if (!r) return fail(KC_ERR_NOMEM, "request");
+    r->t_submit = Clock::now();  // the upload below is part of the latency
     r->kind = 1;
     r->n = n;
     r->nnz = (uint64_t)nnz;
