@@ -303,6 +303,9 @@ int kc_graph_from_edges(const uint32_t *src, const uint32_t *dst, uint64_t m, ui
     if (m) {
         cudaError_t e1 = cudaMemcpy(ds, src, m * 4, cudaMemcpyHostToDevice);
         cudaError_t e2 = cudaMemcpy(dd, dst, m * 4, cudaMemcpyHostToDevice);
+        // the builder's stream does not wait for the legacy one, and a short
+        // copy returns before it is on the device
+        if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(cudaStreamLegacy);
         if (e1 != cudaSuccess || e2 != cudaSuccess) {
             dfree(ds);
             dfree(dd);
