@@ -617,7 +617,7 @@ int kc_graph_set_param(kc_graph *g, const char *name, int64_t value) {
             return fail(KC_ERR_INVALID, "peel.chunk: 0 (by graph size) or a power of two in [256, 2^20]");
         t.peel_chunk = (int)value;
     } else if (k == "peel.spill") {
-        if (value < 0 || value > 3072) return fail(KC_ERR_INVALID, "peel.spill: [0, 3072]");
+        if (value < -1 || value > 3072) return fail(KC_ERR_INVALID, "peel.spill: -1 (by row length) or [0, 3072]");
         t.peel_spill = (int)value;
     } else if (k == "peel.steal") {
         if (value < 1 || value > 64) return fail(KC_ERR_INVALID, "peel.steal: [1, 64]");
