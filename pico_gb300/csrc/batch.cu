@@ -26,6 +26,7 @@
 #include <mutex>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "kc_device.cuh"
@@ -99,7 +100,13 @@ __device__ __forceinline__ unsigned bit_or_zero(unsigned d) {
 //     items' entries as one sequence, 32 x BATCH_U at a time.  The owner of an
 //     entry is counted: the items that start within a window of 32 entries set
 //     one bit each (one reduction), an entry's owner is the number of starts
-//     at or before it;
+//     at or before it.  A round of at most one item per warp, which long chains
+//     and the ends of most cascades consist of, hands nothing out, scans nothing
+//     and looks no owner up, and its short rows are one window (a path of 40,000
+//     vertices 35.7 -> 19.7 ms, the mix 8.6 -> 7.9, 256 small graphs 0.31 ->
+//     0.25, R-MAT 20,011 / 320,000 without allocation 0.78 -> 0.65; the same
+//     branch as a condition ahead of the loop, not an if and else, leaves the
+//     mix at 8.8);
 //   * one barrier per round (the counters of three rounds rotate);
 //   * queues live in shared memory (ids: id_cap, two rings of q_cap ranges for
 //     the round read and the round filled); what does not fit goes to the
@@ -185,8 +192,14 @@ __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
                 r1 = rp[v + 1] - e0;
                 k = (uint32_t)((r1 - r0 + chunk - 1) / chunk);
             }
-            unsigned tot;
-            const unsigned ex = warp_excl_scan(k, lane, tot);
+            unsigned tot, ex;
+            if (__any_sync(KC_FULL_MASK, k > 1)) {
+                ex = warp_excl_scan(k, lane, tot);
+            } else {  // one range each
+                const unsigned m = __ballot_sync(KC_FULL_MASK, k != 0);
+                ex = __popc(m & (le >> 1));
+                tot = __popc(m);
+            }
             unsigned base = 0;
             if (lane == 0 && tot) base = atomicAdd(&cnt[rr % 3], tot);
             base = __shfl_sync(KC_FULL_MASK, base, 0) + ex;
@@ -300,46 +313,37 @@ __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
                 }
                 const unsigned fb_next = fb + total_items;
                 const unsigned long long *slot = ring + (r & 1) * q_cap;
-                const unsigned per = min(32u, (total_items + nwarps - 1) / nwarps);
-                for (;;) {
-                    unsigned i0 = 0;
-                    if (lane == 0) i0 = atomicAdd(&head[r % 3], per);
-                    i0 = __shfl_sync(KC_FULL_MASK, i0, 0);
-                    if (i0 >= total_items) break;
-                    Off rs = 0;
-                    uint32_t len = 0;
-                    const unsigned i = i0 + lane;
-                    if (lane < per && i < total_items) {
-                        const unsigned long long it = i < q_cap ? slot[i] : __ldcg(&F[fb + i]);
-                        rs = (Off)(it >> 24);
-                        len = (uint32_t)(it & 0xffffffull);
-                    }
-                    unsigned total;
-                    const unsigned off = warp_excl_scan(len, lane, total);
-                    rs -= (Off)off;  // entry e of the sequence is at rs + e of its owner
-                    const unsigned start = len && lane ? off : 0x80000000u;  // items have at least one entry
+                // Walks a warp's entries, U windows of 32 at a time: entry e of the
+                // sequence is at rs + e of its owner, the last item with start <= e.
+                // ONE: all of one item, rs the same on every lane.
+                auto walk = [&](auto windows, auto one, Off rs, unsigned start, unsigned total) {
+                    constexpr int U = decltype(windows)::value;
+                    constexpr bool ONE = decltype(one)::value;
                     unsigned before = 0;  // items after the first that start before the window
-                    for (unsigned base = 0; base < total; base += 32 * BATCH_U) {
-                        uint32_t u[BATCH_U];
+                    for (unsigned base = 0; base < total; base += 32 * U) {
+                        uint32_t u[U];
 #pragma unroll
-                        for (int k = 0; k < BATCH_U; k++) {
+                        for (int k = 0; k < U; k++) {
                             const unsigned e = base + k * 32 + lane;
-                            const unsigned starts = __reduce_or_sync(KC_FULL_MASK, bit_or_zero(start - (base + k * 32)));
-                            const unsigned owner = before + __popc(starts & le);
-                            before += __popc(starts);
-                            const Off at = __shfl_sync(KC_FULL_MASK, rs, owner) + (Off)e;
+                            Off at = rs + (Off)e;
+                            if constexpr (!ONE) {
+                                const unsigned starts = __reduce_or_sync(KC_FULL_MASK, bit_or_zero(start - (base + k * 32)));
+                                const unsigned owner = before + __popc(starts & le);
+                                before += __popc(starts);
+                                at = __shfl_sync(KC_FULL_MASK, rs, owner) + (Off)e;
+                            }
                             u[k] = e < total ? __ldcs(&colv[at]) - v0 : NO_LVL;
                         }
                         // Decrement the unclaimed neighbours.  The decrement that
                         // moves a neighbour from L + 1 to L claims it, at core L,
                         // and queues its row; `above` tracks the smallest residual
                         // degree left above L (smaller old degrees wrap around).
-                        unsigned claims = 0, old[BATCH_U];
+                        unsigned claims = 0, old[U];
 #pragma unroll
-                        for (int k = 0; k < BATCH_U; k++)
+                        for (int k = 0; k < U; k++)
                             if (u[k] != NO_LVL && is_claimed<SMEM>(bits, flags, u[k])) u[k] = NO_LVL;
 #pragma unroll
-                        for (int k = 0; k < BATCH_U; k++) {
+                        for (int k = 0; k < U; k++) {
                             old[k] = 0;
                             if (u[k] != NO_LVL) {
                                 if (sizeof(DegT) == 2) {
@@ -351,7 +355,7 @@ __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
                             }
                         }
 #pragma unroll
-                        for (int k = 0; k < BATCH_U; k++) {
+                        for (int k = 0; k < U; k++) {
                             above = min(above, old[k] - (L + 2));
                             if (old[k] == L + 1) {
                                 claims |= 1u << k;
@@ -367,11 +371,41 @@ __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
                         while (__any_sync(KC_FULL_MASK, claims != 0)) {
                             uint32_t v = 0;
 #pragma unroll
-                            for (int k = BATCH_U - 1; k >= 0; k--)
+                            for (int k = U - 1; k >= 0; k--)
                                 if ((claims >> k) & 1u) v = u[k];
                             enqueue(claims != 0, v, r + 1, fb_next);
                             claims &= claims - 1;
                         }
+                    }
+                };
+                const unsigned per = min(32u, (total_items + nwarps - 1) / nwarps);
+                if (per == 1) {
+                    if ((tid >> 5) < total_items) {
+                        const unsigned i = tid >> 5;
+                        const unsigned long long it = i < q_cap ? slot[i] : __ldcg(&F[fb + i]);
+                        const unsigned len = (unsigned)(it & 0xffffffull);
+                        if (len <= 32) walk(std::integral_constant<int, 1>{}, std::true_type{}, (Off)(it >> 24), 0u, len);
+                        else walk(std::integral_constant<int, 4>{}, std::true_type{}, (Off)(it >> 24), 0u, len);
+                    }
+                } else {
+                    for (;;) {
+                        unsigned i0 = 0;
+                        if (lane == 0) i0 = atomicAdd(&head[r % 3], per);
+                        i0 = __shfl_sync(KC_FULL_MASK, i0, 0);
+                        if (i0 >= total_items) break;
+                        Off rs = 0;
+                        uint32_t len = 0;
+                        const unsigned i = i0 + lane;
+                        if (lane < per && i < total_items) {
+                            const unsigned long long it = i < q_cap ? slot[i] : __ldcg(&F[fb + i]);
+                            rs = (Off)(it >> 24);
+                            len = (uint32_t)(it & 0xffffffull);
+                        }
+                        unsigned total;
+                        const unsigned off = warp_excl_scan(len, lane, total);
+                        rs -= (Off)off;  // entry e of the sequence is at rs + e of its owner
+                        const unsigned start = len && lane ? off : 0x80000000u;  // items have at least one entry
+                        walk(std::integral_constant<int, BATCH_U>{}, std::false_type{}, rs, start, total);
                     }
                 }
                 __syncthreads();
