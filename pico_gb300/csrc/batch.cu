@@ -271,6 +271,14 @@ __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
                     }
                 }
                 if (!__any_sync(KC_FULL_MASK, claims != 0)) continue;
+                if (L == 0 && lev == 0) {
+                    // vertices without a row: nothing to queue
+                    for (; claims; claims &= claims - 1) {
+                        const unsigned j = __ffs(claims) - 1;
+                        A.core[v0 + 8 * (b + (j >> 3) * nthreads + tid) + (j & 7)] = 0;
+                    }
+                    continue;
+                }
                 unsigned tot;
                 unsigned pos = warp_excl_scan(__popc(claims), lane, tot);
                 unsigned base = 0;
