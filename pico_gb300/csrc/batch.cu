@@ -116,10 +116,14 @@ __device__ __forceinline__ unsigned bit_or_zero(unsigned d) {
 // 38.0 -> 8.6 ms, 256 graphs of up to 3,162 vertices 0.96 -> 0.29 ms.  On
 // Erdos-Renyi graphs alone an SM walks 1.95 G row entries/s, 2.6 instructions
 // each, the issue slots 62% busy.
-template <typename DegT, bool SMEM>
+// WIDE: 16-bit degrees up to 65,534 and no mark; the scan takes claimed vertices
+// out by the claim bits of the group, a byte beside its degrees.
+template <typename DegT, bool SMEM, bool WIDE = false>
 __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
+    static_assert(!WIDE || (SMEM && sizeof(DegT) == 2), "wide degrees are 16-bit ones in shared memory");
     using Off = typename OffOf<SMEM>::type;  // entry offset within the graph
-    constexpr unsigned MARK = 1u << (8 * sizeof(DegT) - 1);  // degrees are below it
+    // degrees are below it
+    constexpr unsigned MARK = WIDE ? 0xffffu : 1u << (8 * sizeof(DegT) - 1);
     extern __shared__ __align__(16) unsigned char smem[];
     // cnt[r % 3]: items of round r; head[r % 3]: next item to take in round r
     __shared__ unsigned int gi_sh, idcnt, cnt[3], head[3], minlev[2];
@@ -224,6 +228,14 @@ __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
                     if (c >= groups) continue;
                     uint4 *p = reinterpret_cast<uint4 *>(deg) + c * (sizeof(DegT) / 2);
                     uint4 x = SMEM ? p[0] : __ldcg(p);
+                    if constexpr (WIDE) {
+                        const unsigned gone = reinterpret_cast<const uint8_t *>(bits)[c];
+                        auto two = [&](int j) { return ((gone >> j) & 1u) * 0xffffu | ((gone >> (j + 1)) & 1u) * 0xffff0000u; };
+                        x.x |= two(0);
+                        x.y |= two(2);
+                        x.z |= two(4);
+                        x.w |= two(6);
+                    }
                     unsigned low = 0;  // vertices at or below L
                     if constexpr (sizeof(DegT) == 2) {
                         unsigned gm = __vimin3_u16x2(x.x, x.y, __vimin3_u16x2(x.z, x.w, x.w));
@@ -236,7 +248,7 @@ __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
                                     w[j / 2] |= MARK << (16 * (j & 1));
                                 }
                             }
-                            p[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                            if (!WIDE) p[0] = make_uint4(w[0], w[1], w[2], w[3]);
                             gm = __vimin3_u16x2(w[0], w[1], __vimin3_u16x2(w[2], w[3], w[3]));
                         }
                         min2 = __vimin3_u16x2(min2, gm, gm);
@@ -369,9 +381,9 @@ __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
                                 claims |= 1u << k;
                                 if (SMEM) atomicOr(&bits[u[k] >> 5], 1u << (u[k] & 31));
                                 else flags[u[k]] = 1;
-                                if (sizeof(DegT) == 2)
+                                if (sizeof(DegT) == 2 && !WIDE)
                                     atomicOr(reinterpret_cast<unsigned int *>(deg) + (u[k] >> 1), MARK << ((u[k] & 1) * 16));
-                                else
+                                else if (!WIDE)
                                     atomicOr(reinterpret_cast<unsigned int *>(deg) + u[k], MARK);
                                 A.core[v0 + u[k]] = L;
                             }
@@ -420,7 +432,7 @@ __global__ void __launch_bounds__(1024, 1) batch_peel(BatchArgs A) {
                 fb = fb_next;
                 r++;
             }
-            // (old degrees of vertices claimed meanwhile have the top bit set)
+            // (old degrees of vertices claimed meanwhile have the top bit set, or are at most L)
             if (L + 2 < MARK && above < MARK - (L + 2)) my_min = min(my_min, above + L + 1);
             my_min = __reduce_min_sync(KC_FULL_MASK, my_min);
             if (lane == 0 && my_min != NO_LVL) atomicMin(&minlev[lev & 1], my_min);
@@ -510,8 +522,8 @@ struct BatchConfig {
 };
 
 // Graphs of one size class run with the same kernel and launch shape.
-enum : int { BATCH_U16 = 0, BATCH_U32 = 1, BATCH_GLOBAL = 2 };
-constexpr int BATCH_CLASSES = 6;
+enum : int { BATCH_U16 = 0, BATCH_U32 = 1, BATCH_GLOBAL = 2, BATCH_WIDE = 3 };
+constexpr int BATCH_CLASSES = 7;
 struct BatchClass {
     int kind = BATCH_U16;  // degree type and place
     int index = 0;         // work counter of the class
@@ -570,12 +582,12 @@ static void free_classes(kc_batch *b) {
     b->planned = false;
 }
 
-// Raises the dynamic shared-memory limit of batch_peel<DegT, SMEM> on the
+// Raises the dynamic shared-memory limit of batch_peel<DegT, SMEM, WIDE> on the
 // current device to the opt-in maximum, once per device.  The limit is never
 // lowered afterwards, so a launch planned for one size stays valid whatever
 // other launches of the same kernel (a later plan, the allocation-free entry
 // point, another host thread) need.
-template <typename DegT, bool SMEM>
+template <typename DegT, bool SMEM, bool WIDE = false>
 static int batch_smem_limit() {
     static std::mutex mu;
     static bool done[64] = {};
@@ -584,7 +596,7 @@ static int batch_smem_limit() {
     if (dev < 0 || dev >= 64) return fail(KC_ERR_INVALID, "device %d out of range", dev);
     std::lock_guard<std::mutex> lk(mu);
     if (done[dev]) return KC_OK;
-    auto fn = batch_peel<DegT, SMEM>;
+    auto fn = batch_peel<DegT, SMEM, WIDE>;
     int optin = 0;
     KC_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cudaFuncAttributes fa;
@@ -594,11 +606,11 @@ static int batch_smem_limit() {
     return KC_OK;
 }
 
-template <typename DegT, bool SMEM>
+template <typename DegT, bool SMEM, bool WIDE = false>
 static int class_grid(int threads, size_t smem, int sms, int *grid) {
-    auto fn = batch_peel<DegT, SMEM>;
+    auto fn = batch_peel<DegT, SMEM, WIDE>;
     // whatever the size: 48 KB without the opt-in count the static variables too
-    KC_TRY((batch_smem_limit<DegT, SMEM>()));
+    KC_TRY((batch_smem_limit<DegT, SMEM, WIDE>()));
     int occ = 0;
     KC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem));
     if (occ < 1) return fail(KC_ERR_UNSUPPORTED, "batch kernel (%d threads, %zu B shared) cannot be resident", threads, smem);
@@ -607,10 +619,14 @@ static int class_grid(int threads, size_t smem, int sms, int *grid) {
 }
 
 // Size classes: graphs of at most small_n vertices; then, while the degrees
-// fit 16 bits, graphs of which four, two or one fit the shared memory of an SM
+// fit 15 bits, graphs of which four, two or one fit the shared memory of an SM
 // (large_threads / 4, / 2 and / 1 threads each: at 64 registers a thread an SM
 // holds 1,024 threads, and the barriers of several CTAs overlap where one CTA
-// of all the threads would wait); 32-bit degrees; global memory.
+// of all the threads would wait); 32-bit degrees; 16-bit ones without the mark
+// for what is too large for those (more than about 53,000 vertices) and has a hub
+// of 32,768 to 65,534 entries; global memory.  304 graphs of 100,000 vertices,
+// average degree 1 / 4 / 16, with a hub of 40,000 entries: 1.90 / 3.57 / 5.78 ms in
+// global memory, 1.40 / 2.32 / 3.13 with wide degrees.
 static int plan(kc_batch *b) {
     free_classes(b);
     int dev = b->g->device, smem_max = 0, smem_sm = 0;
@@ -634,21 +650,23 @@ static int plan(kc_batch *b) {
     for (uint32_t i = 0; i < b->G; i++) {
         const uint32_t n = b->vbase[i + 1] - b->vbase[i];
         const bool fits16 = b->maxdeg[i] < 32768u;  // the top bit is the scan's mark
+        const bool fits_wide = b->maxdeg[i] < 65535u;
         int k;
-        if (b->nnz[i] >= (1ull << 31)) k = 5;  // 32-bit entry offsets in the shared-memory kernels
+        if (b->nnz[i] >= (1ull << 31)) k = 6;  // 32-bit entry offsets in the shared-memory kernels
         else if (fits16 && n <= small_n) k = 0;
-        else if (!b->cfg.large_shared) k = 5;
+        else if (!b->cfg.large_shared) k = 6;
         else if (fits16 && n <= mid_n[0]) k = 1;
         else if (fits16 && n <= mid_n[1]) k = 2;
         else if (fits16 && n <= large_u16) k = 3;
         else if (n <= large_u32) k = 4;
-        else k = 5;
+        else if (fits_wide && n <= large_u16) k = 5;
+        else k = 6;
         cls[k].order.push_back(i);
     }
     for (int k = 0; k < BATCH_CLASSES; k++) {
         BatchClass &c = cls[k];
         if (c.order.empty()) continue;
-        c.kind = k <= 3 ? BATCH_U16 : k == 4 ? BATCH_U32 : BATCH_GLOBAL;
+        c.kind = k <= 3 ? BATCH_U16 : k == 4 ? BATCH_U32 : k == 5 ? BATCH_WIDE : BATCH_GLOBAL;
         std::stable_sort(c.order.begin(), c.order.end(),
                          [&](uint32_t x, uint32_t y) { return b->nnz[x] > b->nnz[y]; });
         // shrink the shared arrays to the largest graph of the class
@@ -657,7 +675,7 @@ static int plan(kc_batch *b) {
         c.smem_n = c.kind == BATCH_GLOBAL ? 0u : std::max<uint32_t>(32, (nmax + 31) & ~31u);
         c.threads = k == 0 ? b->cfg.small_threads : b->cfg.large_threads;
         if (k == 1 || k == 2) c.threads = std::max(64, c.threads / (k == 1 ? 4 : 2) & ~31);
-        const size_t own = batch_graph_bytes(c.smem_n, c.kind == BATCH_U16 ? 2 : 4);
+        const size_t own = batch_graph_bytes(c.smem_n, c.kind == BATCH_U16 || c.kind == BATCH_WIDE ? 2 : 4);
         c.id_cap = (unsigned)c.threads;
         c.q_cap = (unsigned)c.threads / 2;
         while (own + batch_queue_bytes(c.q_cap, c.id_cap) > budget && c.q_cap) c.q_cap /= 2;
@@ -667,6 +685,7 @@ static int plan(kc_batch *b) {
         int rc;
         if (c.kind == BATCH_U16) rc = class_grid<uint16_t, true>(c.threads, c.smem_bytes, b->g->sm_count, &grid);
         else if (c.kind == BATCH_U32) rc = class_grid<uint32_t, true>(c.threads, c.smem_bytes, b->g->sm_count, &grid);
+        else if (c.kind == BATCH_WIDE) rc = class_grid<uint16_t, true, true>(c.threads, c.smem_bytes, b->g->sm_count, &grid);
         else rc = class_grid<uint32_t, false>(c.threads, c.smem_bytes, b->g->sm_count, &grid);
         if (rc) return rc;
         c.grid = (int)std::min<size_t>((size_t)grid, c.order.size());
@@ -718,6 +737,7 @@ static int launch_all(kc_batch *b, cudaStream_t s) {
         A.id_cap = c.id_cap;
         if (c.kind == BATCH_U16) batch_peel<uint16_t, true><<<c.grid, c.threads, c.smem_bytes, cs>>>(A);
         else if (c.kind == BATCH_U32) batch_peel<uint32_t, true><<<c.grid, c.threads, c.smem_bytes, cs>>>(A);
+        else if (c.kind == BATCH_WIDE) batch_peel<uint16_t, true, true><<<c.grid, c.threads, c.smem_bytes, cs>>>(A);
         else batch_peel<uint32_t, false><<<c.grid, c.threads, c.smem_bytes, cs>>>(A);
         KC_CUDA(cudaGetLastError());
         if (k > 0) {
