@@ -495,10 +495,13 @@ __global__ void __launch_bounds__(STAGE ? 1024 : PART_THREADS) part_rows(const u
 // Rows per bucket for n vertices (as a shift), or -1 where partitioning does not
 // apply: fewer edges than PART_MIN_EDGES (the atomics' lines stay in L2 and the
 // launches cost more; R-MAT 16, 1.05 M edges: 0.54 ms without, 0.52 with), more rows than the
-// buckets cover, or more entries than a 32-bit offset within a bucket holds.
-constexpr uint64_t PART_MIN_EDGES = 1u << 20;
+// buckets cover, more than PART_MAX_ROWS rows per edge (the tiles' row counters
+// then outweigh the edges: 2^26 vertices, 2^20 edges de-duplicated 2.5 ms with,
+// 2.0 without; 2^22 edges sorted 1.7 with, 2.1 without), or more entries than a
+// 32-bit offset within a bucket holds.
+constexpr uint64_t PART_MIN_EDGES = 1u << 20, PART_MAX_ROWS = 16;
 static int part_shift(uint64_t m, uint32_t n) {
-    if (m < PART_MIN_EDGES || 2 * m >= 0xffffffffull) return -1;
+    if (m < PART_MIN_EDGES || 2 * m >= 0xffffffffull || n > PART_MAX_ROWS * m) return -1;
     int shift = 6;
     while (shift < PART_MAX_SHIFT && ((n - 1) >> shift) + 1 > PART_MAX_BUCKETS / 2) shift++;
     return ((n - 1) >> shift) + 1 <= PART_MAX_BUCKETS ? shift : -1;
@@ -1579,8 +1582,9 @@ int build_csr_from_edges(Graph *g, const uint32_t *d_src, const uint32_t *d_dst,
     cudaMemsetAsync(deg, 0, ((uint64_t)n + 1) * 4, s);
     cudaMemsetAsync(err, 0, 4, s);
     // partitioned where the order within a row is free and there is room for
-    // the pairs (16 bytes per edge) and the tiles' row shares (6 bytes per row of a
-    // bucket and tile: 0.8 bytes per edge with 2,048 rows, at most 6)
+    // the pairs (16 bytes per edge) and the tiles' row shares, 6 bytes x (2 m /
+    // PART_TILE + buckets) x rows per bucket: 1.1 bytes per edge on R-MAT 22, up to
+    // 102 where rows outnumber edges by PART_MAX_ROWS
     PartPlan plan{};
     uint2 *pairs = nullptr;
     plan.shift = part_shift(m, n);
