@@ -330,7 +330,7 @@ int kc_graph_from_mtx(const char *path, int mode, int device, kc_graph **out) {
     return rc;
 }
 
-// Largest degree and number of 32-wide virtual nodes of a CSR in host memory.
+// A graph from a CSR in host or device memory.
 static int from_csr_common(const int64_t *rowptr, const uint32_t *col, uint32_t n, int device, kc_graph **out,
                            cudaMemcpyKind kind) {
     NvtxRange nvtx_("kc_graph_from_csr");

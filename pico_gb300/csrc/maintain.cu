@@ -545,7 +545,6 @@ __global__ void endpoints(const uint32_t *__restrict__ src, const uint32_t *__re
     }
 }
 
-// Temporary device arrays freed on scope exit.
 // Scratch arrays of one call, freed when the call returns (after the call's
 // stream has finished with them, so an early error return cannot free memory
 // that a launched kernel still uses).

@@ -22,13 +22,15 @@
 //     from the host, or uses a block-local queue guarded by a device assert).
 //     A decrement that finds deg <= L is undone (the reference's clamp,
 //     peelone.cu:80-86 / peelone-dyn.cc:95-98); values above L feed the
-//     next-level minimum.  Each CTA keeps at most SPILL_T queued items in
-//     shared memory; the rest go to a global queue that idle CTAs steal from.
+//     next-level minimum.  Each CTA keeps a limited number of queued items in
+//     shared memory (SPILL_AUTO below); the rest go to a global queue that idle
+//     CTAs steal from.
 //   * level skipping: the next level is the smallest residual degree seen,
 //     not L+1, so empty levels cost nothing.
 // Work accounting instead of a grid barrier: every level has a counter of
 // outstanding credits (one per CTA until its list is scanned and its queue
-// drained, plus every item put on the global queue).  A level ends when the
+// drained, plus every item put on the global queue until a CTA takes it; a CTA
+// that was idle keeps one for itself and hands the others back).  A level ends when the
 // counter is zero; the CTA that brought it there announces the next level.
 // Against one alive list shared by all CTAs (a reservation per warp on one
 // counter, rewritten every level) and waits on the credit count itself:

@@ -558,8 +558,8 @@ int kc_server_submit_decompose(kc_server *S, const int64_t *rowptr, const uint32
     r->kind = 1;
     r->n = n;
     r->nnz = (uint64_t)nnz;
-    // device footprint: CSR, core, batch queues, degrees and alive lists,
-    // with headroom
+    // device footprint: CSR, core, row-range queue, degrees, and the peel's
+    // lists and queues of a graph that runs alone, with headroom
     r->need = 3 * (8ull * (n + 1) + 4ull * nnz) + 24ull * n + (1ull << 20);
     if (!upload(S, r, rowptr, col)) {
         r->rowptr.assign(rowptr, rowptr + n + 1);
