@@ -838,7 +838,7 @@ static int order_range(OrderBuild &B, uint32_t row0, uint32_t rows) {
         const bool last = p + 1 == passes;
         uint32_t *col = g->col ? g->col + B.done : nullptr;
         if (p == 0) {
-            cudaMemsetAsync(B.state, 0, 16, s);
+            if (!all) cudaMemsetAsync(B.state, 0, 16, s);
             order_hist<true><<<ctas, ORDER_THREADS, hist_sm, s>>>(P, all ? reinterpret_cast<unsigned int *>(B.state + 1) : nullptr);
             order_scan<<<scan_ctas, 1024, 0, s>>>(P, ctas, B.state);
             cudaMemcpyAsync(h, B.state, 16, cudaMemcpyDeviceToHost, s);
@@ -888,6 +888,8 @@ static int build_in_order(Graph *g, const uint32_t *d_src, const uint32_t *d_dst
     KC_TRY(dalloc(&B.hist, (B.stretches + 1) << ORDER_MAX_BITS, "digit counts"));
     KC_TRY(dalloc(&B.state, 2, "entry count"));
     KC_TRY(dalloc(&B.deg, (uint64_t)n + 1, "degrees"));
+    // ahead of the larger one, so that the first kernel follows it at once
+    cudaMemsetAsync(B.state, 0, 16, s);
     cudaMemsetAsync(B.deg, 0, ((uint64_t)n + 1) * 4, s);
     KC_TRY(order_range(B, 0, n));
     KC_TRY(exclusive_scan_u32_i64(B.deg, g->rowptr, n, s));
