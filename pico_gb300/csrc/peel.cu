@@ -89,7 +89,7 @@ constexpr unsigned PROBE_MIN = 512;
 // 1.74 / 3.66 / 1.15, Barabasi-Albert 10^6 x 8 and 500,000 x 16 1.56 and 1.27 /
 // 2.13 and 2.48 / 1.21 and 1.29; what has work everywhere is the same or pays for
 // the look at the count: uniform random 65,536 0.227 -> 0.223, R-MAT 22 5.25 ->
-// 5.30, R-MAT 25 with a planted core 20.8 -> 21.0.  A limit of 8 items doubles the
+// 5.29, R-MAT 25 with a planted core 20.8 -> 20.9.  A limit of 8 items doubles the
 // grids' times; a lower line than every CTA is slower on the grids and the cubes,
 // twice as high a line on the uniform random graphs (10^6 x 3 0.17 -> 0.50).
 constexpr unsigned SPILL_AUTO = ~0u, SPILL_ENTRIES = 16384, SPILL_MIN = 4, SPILL_MAX = 1024, SPILL_IDLE = 16;
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
     __shared__ unsigned long long wait_t0;
     __shared__ unsigned int withheld;
     __shared__ unsigned int rounds_sh;
-    __shared__ unsigned int idle_sh;  // when the last round began, an idle CTA had nothing to take
+    __shared__ unsigned int work_sh;  // CTAs at work and items nobody had taken when the last round began
     __shared__ unsigned long long mode_ns[4], mode_t0;  // trace: time per mode in this level
     __shared__ int prev_mode;
     __shared__ unsigned int bal_off[BAL ? NT + 1 : 1];  // balanced rounds: item offsets,
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
             claimed_any = 0;
             wait_t0 = 0;
             rounds_sh = 0;
-            idle_sh = 0;
+            work_sh = G;
             if (A.trace) {
                 mode_ns[0] = mode_ns[1] = mode_ns[2] = mode_ns[3] = 0;
                 mode_t0 = global_ns();
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
             {
                 // read now, used by the next round, so that nobody waits for it (the low word is all of it)
                 const unsigned at_work =
-                    tid == NT - 32 ? ld_relaxed(reinterpret_cast<unsigned *>(&ctl->pending[s].left)) : 0u;
+                    tid == 0 ? ld_relaxed(reinterpret_cast<unsigned *>(&ctl->pending[s].left)) : 0u;
                 // the CTA queue's head once this round's items are taken (the
                 // spill threshold counts the items queued behind it)
                 unsigned round_head = q_head;
@@ -883,7 +883,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                                     KC_FULL_MASK, push ? (unsigned)min(cr1[k] - cr0[k], (int64_t)RANGE_LEN) : 0u);
                                 const unsigned halves = (sum > 32 * cnt) + (sum > 128 * cnt);
                                 keep = min(SPILL_MAX, max(SPILL_MIN, (SPILL_ENTRIES >> halves) * cnt / max(sum, 1u)));
-                                if (idle_sh) keep = min(keep, SPILL_IDLE);
+                                if (work_sh < G) keep = min(keep, SPILL_IDLE);
                             }
                             unsigned slot_lo = 0, slot_hi = 0;
                             int spill = 0;
@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) peel_kernel(PeelArgs A) {
                 local_min = __reduce_min_sync(KC_FULL_MASK, local_min);
                 if (lane == 0 && local_min != NO_LEVEL) atomicMin(&min_sh, local_min);
                 if (lane == 0 && nit) claimed_any = 1;
-                if (tid == NT - 32) idle_sh = at_work < G;
+                if (tid == 0) work_sh = at_work;
                 if (A.trace && lane == 0 && wclaims) atomicAdd(&claims_sh, wclaims);
             }
             __syncthreads();
