@@ -343,7 +343,7 @@ int kc_graph_from_segment(const kc_graph *g, uint32_t lo, uint32_t hi, kc_graph 
  * allows (cudaMemGetInfo minus hbm_reserve_bytes minus what admitted requests
  * may still allocate); a lane packs all admissible waiting requests (up to
  * max_batch_graphs / max_batch_bytes) into one batched launch.  Inputs are
- * copied at submission: graphs of 256 KB and more to the device, as long as
+ * copied at submission: graphs of 768 KB and more to the device, as long as
  * all admitted requests fit in decompose_slots * max_batch_bytes and in the
  * free memory, else to host memory.  Latency = submission (the start of the
  * submitting call, so with that copy) to result on the host. */

@@ -78,8 +78,12 @@ using Clock = std::chrono::steady_clock;
 // 80-100 GB/s, where a copy in fresh host memory runs at 15 GB/s and the lane
 // then packs it in another and uploads that.  32 graphs of 78 MB: submitted in
 // 1.7 instead of 5.0 ms, served beside two updates in 8.7 instead of 11.8 ms.
-// Below the line the device calls (about 40 us a request) are the larger cost.
-constexpr uint64_t UPLOAD_MIN = 256u << 10;
+// Below the line the device calls (about 75 us a request) are the larger cost.
+// Requests of 260 / 400 KB x 128, 600 / 800 / 1,000 KB x 64 and 2 MB x 32, all sent
+// to the device against none: 9.8 / 9.9 / 5.3 / 5.4 / 5.6 / 3.9 ms against 3.3 / 5.0
+// / 3.9 / 5.0 / 6.5 / 6.9 (beside two updates 10.2 / 10.3 / 6.4 / 6.5 / 6.8 / 7.1
+// against 5.7 / 6.3 / 7.5 / 8.3 / 9.3 / 8.9).
+constexpr uint64_t UPLOAD_MIN = 768u << 10;
 
 struct Request {
     uint64_t ticket = 0;
