@@ -17,8 +17,8 @@ Printed JSON line (rank 0):
              (independent graph handles), so one step's upload overlaps the
              previous steps' decompositions, and these graphs run the peel on
              one CTA per SM so that two decompositions share the GPU (a peel
-             alone is latency-bound: 28.0 ms on half the CTAs against 22.7 ms
-             on all, but two at once take 17.8 ms each); serial_value: one
+             alone is latency-bound: 27.9 ms on half the CTAs against 20.1 ms
+             on all, but two at once take 16.7 ms each); serial_value: one
              thread and the default grid;
              the same K steps as value, the pipeline's fill (the first upload,
              which overlaps nothing) inside the timed region;
